@@ -44,6 +44,13 @@ __device__ __forceinline__ uint32_t mix32(uint64_t x) {
 
 // Random initial rows (the reference's initialize_graph, :158-166, seeded
 // instead of clock-seeded) with exact distances, sorted, repeats removed.
+// Bound by the random row gathers. Rows above kInitLaneDim are scored by the
+// whole warp (at 250K x 960, K = 64: 6.2 ms against 36.8 ms for a lane per
+// row, whose 1,920-byte rows are 120 scattered loads in turn); narrower ones by
+// a lane each, which needs no shuffle trees (200K x 136: 0.94 ms against 1.55 ms;
+// equal at 256 dims, and 1.35 against 1.14 ms at 100K x 384).
+constexpr uint32_t kInitLaneDim = 256;
+
 __global__ void __launch_bounds__(128)
     k_init(const __half* __restrict__ data, uint32_t n, uint32_t dim, uint32_t K, uint64_t seed,
            uint64_t* __restrict__ nb) {
@@ -60,13 +67,34 @@ __global__ void __launch_bounds__(128)
         keys[t] = (uint64_t)v;
       }
     }
-    // one neighbour row per lane, in the reference's lane order (row_dist)
     const __half* q = data + (size_t)u * dim;
+    if (dim > kInitLaneDim) {
+      // the whole warp scores four rows at a time: coalesced row reads
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      if (keys[t] != kEmpty) {
-        const uint32_t v = (uint32_t)keys[t];
-        keys[t] = make_key(row_dist(q, data + (size_t)v * dim, dim), v, true);
+      for (int t = 0; t < 4; ++t) {
+        for (uint32_t i = 0; i < 32 && 32 * t + i < K; i += 4) {
+          uint32_t ids[4];
+          float o[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const uint32_t v = __shfl_sync(kFull, (uint32_t)keys[t], (int)i + r);
+            ids[r] = 32 * t + i + r < K ? v : kInv;
+          }
+          if (dim == 960) warp_dist4<960>(q, data, dim, ids, o, lane);
+          else warp_dist4(q, data, dim, ids, o, lane);
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if ((uint32_t)lane == i + r && ids[r] != kInv) keys[t] = make_key(o[r], ids[r], true);
+        }
+      }
+    } else {
+      // one neighbour row per lane, in the reference's lane order (row_dist)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (keys[t] != kEmpty) {
+          const uint32_t v = (uint32_t)keys[t];
+          keys[t] = make_key(row_dist(q, data + (size_t)v * dim, dim), v, true);
+        }
       }
     }
     warp_sort_keys<4>(keys, lane);

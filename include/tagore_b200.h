@@ -24,11 +24,11 @@ enum {
   TAGORE_ETIMEOUT = 5  /* a bounded wait ran out */
 };
 
-/* kNN join modes. CHOSEN: tensor-core screen + exact re-rank where the row
- * width allows (one tile for 16..128 dims in steps of 16; the tile
- * accumulated over 64-dim blocks for 129..1024 dims in steps of 8), the
- * learned screen otherwise; PLAIN: every pair in exact FP32; LEARNED: the
- * learned screen at any width. */
+/* kNN join modes. CHOSEN: tensor-core screen + exact re-rank for rows up to
+ * 1024 dims (one tile up to 128 dims, the tile accumulated over 64-dim blocks
+ * from there; widths of 4 mod 8 on a zero-padded copy), the learned screen for
+ * wider rows; PLAIN: every pair in exact FP32; LEARNED: the learned screen at
+ * any width. */
 enum { TAGORE_KNN_CHOSEN = 0, TAGORE_KNN_PLAIN = 1, TAGORE_KNN_LEARNED = 2 };
 
 /* learn_flags of TagoreKnnParams (for measuring the screen against itself):

@@ -34,7 +34,8 @@ struct Work {
 
 int join_tc(const Work& w, cudaStream_t s);
 // Row widths the tensor-core join takes (one 128-row tile of K-major FP16).
-inline bool tc_supported(uint32_t dim) { return dim >= 16 && dim <= 128 && dim % 16 == 0; }
+// TMA wants row strides that are multiples of 16 bytes, hence of 8 halves.
+inline bool tc_supported(uint32_t dim) { return dim >= 8 && dim <= 128 && dim % 8 == 0; }
 // Wider rows: the Gram tile accumulated over 64-half column blocks.
 int join_tc_wide(const Work& w, cudaStream_t s);
 inline bool tc_wide_supported(uint32_t dim) { return dim > 128 && dim <= 1024 && dim % 8 == 0; }

@@ -5,7 +5,7 @@
 // join list (<= 128 FP16 rows):
 //   1. TMA tile::gather4 copies the rows into a K-major 128-byte-swizzled tile
 //      X in shared memory (box 64 halves x 1 row, four rows per copy);
-//   2. one thread issues D/16 tcgen05.mma.kind::f16 (M = N = 128, K = 16), X as
+//   2. one thread issues ceil(D/16) tcgen05.mma.kind::f16 (M = N = 128, K = 16), X as
 //      both operands, so TMEM holds the Gram tile X X^T in FP32;
 //   3. each thread owns one row: it reads its TMEM lane, forms the screened
 //      distance n_r + n_c - 2 g_rc from exact FP32 norms, and keeps its
@@ -136,12 +136,6 @@ __device__ __forceinline__ void fma2_m2(float g0, float g1, float h0, float h1, 
       : "f"(g0), "f"(g1), "f"(h0), "f"(h1), "f"(-2.0f));
 }
 
-// Chunk j (4 halves) of row r inside a swizzled tile.
-__device__ __forceinline__ uint2 tile_chunk(const Tile& t, uint32_t r, uint32_t j) {
-  const uint32_t blk = j >> 4, unit = ((j & 15u) >> 1) ^ (r & 7u), half8 = j & 1u;
-  return *reinterpret_cast<const uint2*>(&t.x[blk][r][unit * 16 + half8 * 8]);
-}
-
 // Chunks 2p and 2p+1 of row r (one 16-byte unit of the swizzled tile).
 __device__ __forceinline__ uint4 tile_pair(const Tile& t, uint32_t r, uint32_t p) {
   return *reinterpret_cast<const uint4*>(&t.x[p >> 3][r][((p & 7u) ^ (r & 7u)) * 16]);
@@ -153,25 +147,11 @@ __device__ __forceinline__ float tile_dist(const Tile& t, uint32_t ra, uint32_t 
   if constexpr (D == 128) {
     return dist128_pairs([&](int p, int w) { return tile_pair(t, w ? rb : ra, (uint32_t)p); });
   } else if constexpr (D > 0) {
-    return serial_dist<D>([&](int j, int w) { return tile_chunk(t, w ? rb : ra, (uint32_t)j); });
+    return dist_pairs_fixed<D / 8>(
+        [&](uint32_t u, int w) { return tile_pair(t, w ? rb : ra, u); });
   } else {
-    float x[32], y[32];
-#pragma unroll
-    for (int l = 0; l < 32; ++l) {
-      x[l] = 0.0f;
-      y[l] = 0.0f;
-    }
-    for (uint32_t j = 0; j < dim / 4; ++j)
-      chunk_acc(tile_chunk(t, ra, j), tile_chunk(t, rb, j), x[j & 31], y[j & 31]);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-      for (int l = 0; l < off; ++l) {
-        x[l] = __fadd_rn(x[l], x[l + off]);
-        y[l] = __fadd_rn(y[l], y[l + off]);
-      }
-    }
-    return __fadd_rn(x[0], y[0]);
+    return dist_pairs_rounds([&](uint32_t u, int w) { return tile_pair(t, w ? rb : ra, u); },
+                             dim >> 3);
   }
 }
 
@@ -304,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   extern __shared__ unsigned char smem_raw[];
   TcSmem& s = *reinterpret_cast<TcSmem*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t ksteps = dim / 16;
+  const uint32_t ksteps = (dim + 15) / 16;  // columns past dim are zero-filled by TMA
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -977,8 +957,8 @@ int join_tc_wide(const Work& w, cudaStream_t s) {
 }
 
 int join_tc(const Work& w, cudaStream_t s) {
-  if (w.dim > 128 || w.dim % 16)
-    return fail(TAGORE_EINVAL, "tensor-core join needs DIM in {16,32,..,128} (got %u)", w.dim);
+  if (!tc_supported(w.dim))
+    return fail(TAGORE_EINVAL, "tensor-core join needs DIM in {8,16,..,128} (got %u)", w.dim);
   if (w.T > 4) return fail(TAGORE_EINVAL, "tensor-core join keeps at most 4 partners per row");
   CUtensorMap map;
   TG_TRY(make_row_map(&map, w.data, w.n, w.dim));

@@ -12,9 +12,11 @@
 //    by target), so the reference's replacement rule for full lists
 //    (:1465-1475, :1697-1707) gives one defined answer;
 //  * the Filter stage is evaluated lazily: a candidate is tested against the
-//    kept neighbours in order and dropped at the first rule that fires, which
-//    keeps exactly the set the reference's round-by-round sweep (:1416-1460)
-//    keeps while computing far fewer distances.
+//    kept neighbours before it and dropped when any rule fires, which keeps
+//    exactly the set the reference's round-by-round sweep (:1416-1460) keeps;
+//    the tests are decided on tensor cores where the screened distance is clear
+//    of the rule's value by its error bound (screen.cuh), and by the exact
+//    distance where it is not.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -24,6 +26,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "knn_shared.cuh"
+#include "screen.cuh"
 
 namespace tagore {
 namespace {
@@ -401,220 +404,178 @@ __device__ __noinline__ void warp_sort_mark(uint32_t* cand, float* dis, uint32_t
   __syncwarp();
 }
 
-// Position of the r-th (0-based) set bit of m; m has more than r set bits.
-// Binary search on population counts: five steps whatever r is.
-__device__ __forceinline__ uint32_t nth_bit(unsigned m, uint32_t r) {
-  uint32_t pos = 0;
-#pragma unroll
-  for (int w = 16; w >= 1; w >>= 1) {
-    const uint32_t c = (uint32_t)__popc(m & ((1u << w) - 1u));
-    const bool skip = r >= c;
-    r -= skip ? c : 0u;
-    m = skip ? m >> w : m;
-    pos += skip ? (uint32_t)w : 0u;
-  }
-  return pos;
-}
-
-// Filter stage, lazily evaluated (see file header). Returns the number of ids
-// the reference stores: one less than its selection steps (:1462, :1623).
-//
-// The lanes work through the sorted list as a queue: each takes the next live
-// candidate and tests it against the kept neighbours in order, one exact
-// thread-serial distance per step, until a rule fires or it has passed them
-// all. The earliest unresolved candidate that has passed is kept, in list
-// order; a candidate further on that had passed must then also pass the new
-// neighbour. Each candidate is thus tested against exactly the neighbours
-// kept before it, as in the sequential filter.
-__device__ uint32_t warp_filter(const uint32_t* cand, const float* cdis, uint32_t len,
-                                uint32_t bid, uint32_t fd, int metric, float thre,
-                                const __half* __restrict__ data, uint32_t dim, uint32_t* sel,
-                                float* seld, int lane, uint32_t* scored = nullptr) {
-  uint32_t first = kInv;
+// Removes the marked entries and the node itself from a sorted, marked list, in
+// place. Returns the entries left; *tail tells whether the list's last entry is
+// among them.
+__device__ __forceinline__ uint32_t warp_compact(uint32_t* cand, float* dis, uint32_t len, uint32_t bid,
+                                 bool* tail, int lane) {
+  const unsigned below = (1u << lane) - 1u;
+  uint32_t m = 0;
+  unsigned ok = 0;
   for (uint32_t base = 0; base < len; base += 32) {
     const uint32_t i = base + lane;
-    const bool ok = i < len && cand[i] != bid && cand[i] != kInv;
-    const unsigned m = __ballot_sync(kFull, ok);
-    if (m) {
-      first = base + __ffs(m) - 1;
-      break;
+    const uint32_t c = i < len ? cand[i] : kInv;
+    const float d = i < len ? dis[i] : 0.0f;
+    ok = __ballot_sync(kFull, c != kInv && c != bid);
+    __syncwarp();  // the chunk is read before an earlier or equal place is written
+    if (c != kInv && c != bid) {
+      const uint32_t p = m + __popc(ok & below);
+      cand[p] = c;
+      dis[p] = d;
     }
-  }
-  if (first == kInv) return 0;
-  if (lane == 0) {
-    sel[0] = cand[first];
-    seld[0] = cdis[first];
+    m += __popc(ok);
   }
   __syncwarp();
-  uint32_t nsel = 1, last_pos = first, rows = 0;
+  *tail = len > 0 && ((ok >> ((len - 1) & 31u)) & 1u);
+  return m;
+}
+
+// Kept neighbours of one node, and the rows of a tile that outlived the kept
+// ones before it: shared memory of one warp.
+struct Kept {
+  uint32_t* id;
+  float *dis, *norm;        // fd each
+  uint32_t* tid;
+  float *tdis, *tnorm;      // 32 each
+  float* tile;              // screen_tile's
+};
+__host__ __device__ inline size_t kept_bytes(uint32_t fd) {
+  return (size_t)fd * 12 + 32 * 12 + kScreenFloats * 4;
+}
+__device__ inline Kept kept_carve(unsigned char* p, uint32_t fd) {
+  Kept k;
+  k.id = reinterpret_cast<uint32_t*>(p);
+  k.dis = reinterpret_cast<float*>(k.id + fd);
+  k.norm = k.dis + fd;
+  k.tid = reinterpret_cast<uint32_t*>(k.norm + fd);
+  k.tdis = reinterpret_cast<float*>(k.tid + 32);
+  k.tnorm = k.tdis + 32;
+  k.tile = k.tnorm + 32;
+  return k;
+}
+
+// The exact test of candidate row c (distance dc) against kept row q (distance
+// dq), by the whole warp. Out of line: it is rarely taken.
+static __device__ __noinline__ bool exact_test(const __half* __restrict__ data, uint32_t dim,
+                                               ScreenRule rule, uint32_t c, float dc, uint32_t q,
+                                               float dq) {
+  const float res = warp_dist(data + (size_t)q * dim, data + (size_t)c * dim, dim,
+                              (int)(threadIdx.x & 31u));
+  return pruned_by(rule.metric, res, dc, dq, rule.thre);
+}
+
+// Filter stage over a compacted list (warp_compact) by one warp. Returns the
+// number of ids the reference stores: one less than its selection steps (:1462,
+// :1623).
+//
+// The list is taken 32 candidates at a time. A tile is first tested against the
+// kept neighbours (16 per screen, stopping when no candidate is left), then its
+// survivors against one another, in list order: each candidate is dropped by a
+// rule that fires against a neighbour kept before it, as in the sequential
+// filter. A repeat of a kept neighbour is dropped too (:1423-1427).
+//
+// Bound by the gathers of the candidates' rows and by instruction issue. Each row
+// is read once per screen; a test costs a fraction of an mma instead of a
+// 2d-byte row and its sum.
+__device__ __forceinline__ uint32_t warp_filter(const uint32_t* cand, const float* cdis,
+                                                uint32_t len, bool tail, uint32_t fd, int metric,
+                                                float thre, const __half* __restrict__ data,
+                                                const float* __restrict__ norms, uint32_t dim,
+                                                const Kept& k, int lane) {
+  const ScreenRule rule{metric, thre, screen_eps(dim)};
   const unsigned below = (1u << lane) - 1u;
-  // lane state: 0 idle, 1 testing against sel[s], 2 passed sel[0, nsel)
-  int st = 0;
-  uint32_t pos = kInv, c = kInv, s = 0;
-  float dc = 0.0f;
-  uint32_t next = first + 1;  // next list position to hand out
-  while (nsel < fd) {
-    unsigned idle = __ballot_sync(kFull, st == 0);
-    while (idle && next < len) {
-      const uint32_t p = next + lane;
-      const unsigned live = __ballot_sync(kFull, p < len && cand[p] != kInv);
-      const uint32_t nlive = __popc(live);
-      const uint32_t take = min(nlive, (uint32_t)__popc(idle));
-      if (st == 0) {
-        const uint32_t r = __popc(idle & below);
-        if (r < take) {
-          pos = next + nth_bit(live, r);
-          c = cand[pos];
-          dc = cdis[pos];
-          s = 0;
-          st = 1;
+  uint32_t nsel = 0, last = 0;
+  for (uint32_t base = 0; base < len && nsel < fd; base += 32) {
+    const uint32_t i = base + lane;
+    uint32_t c = kInv;
+    float dc = 0.0f, nc = 0.0f;
+    if (i < len) {
+      c = cand[i];
+      dc = cdis[i];
+      nc = __ldg(norms + c);
+    }
+    // against the neighbours kept in earlier tiles
+    for (uint32_t k0 = 0; k0 < nsel; k0 += kScreenCols) {
+      const uint2 scr = screen_rows<true>(data, dim, rule, c, nc, dc, k.id + k0, k.norm + k0,
+                                          k.dis + k0, min(kScreenCols, nsel - k0), k.tile);
+      uint32_t amb = scr.x ? 0u : scr.y;
+      bool drop = scr.x != 0;
+      for (unsigned left = __ballot_sync(kFull, amb != 0); left;
+           left = __ballot_sync(kFull, amb != 0)) {
+        const int o = __ffs(left) - 1;
+        const uint32_t q = k0 + __ffs(__shfl_sync(kFull, amb, o)) - 1;
+        const bool f = exact_test(data, dim, rule, __shfl_sync(kFull, c, o),
+                                  __shfl_sync(kFull, dc, o), k.id[q], k.dis[q]);
+        if (lane == o) {
+          drop = f;
+          amb = f ? 0u : amb & (amb - 1u);
         }
       }
-      next = take == nlive ? min(len, next + 32) : next + nth_bit(live, take - 1) + 1;
-      idle = __ballot_sync(kFull, st == 0);
+      if (drop) c = kInv;
+      if (!__any_sync(kFull, c != kInv)) break;
     }
-    if (!__any_sync(kFull, st != 0)) break;
-    if (st == 1) {
-      const uint32_t q = sel[s];
-      if (q == c) {
-        st = 0;  // a repeat of a kept neighbour (:1423-1427)
-      } else {
-        const float res = row_dist(data + (size_t)q * dim, data + (size_t)c * dim, dim);
-        ++rows;
-        if (pruned_by(metric, res, dc, seld[s], thre)) st = 0;
-        else if (++s == nsel) st = 2;
-      }
+    const unsigned alive = __ballot_sync(kFull, c != kInv);
+    const uint32_t ns = __popc(alive);
+    if (ns == 0) continue;
+    __syncwarp();
+    if (c != kInv) {
+      const uint32_t p = __popc(alive & below);
+      k.tid[p] = c;
+      k.tdis[p] = dc;
+      k.tnorm[p] = nc;
     }
-    while (true) {
-      const uint32_t key = st != 0 ? pos : kInv;
-      const uint32_t mn = __reduce_min_sync(kFull, key);
-      if (mn == kInv) break;
-      const int o = __ffs(__ballot_sync(kFull, key == mn)) - 1;
-      if (__shfl_sync(kFull, st, o) != 2) break;
-      if (lane == o) {
-        sel[nsel] = c;
-        seld[nsel] = dc;
-        st = 0;
-      }
-      __syncwarp();
-      ++nsel;
-      last_pos = mn;
-      if (nsel == fd) break;
-      if (st == 2) st = 1;  // s == nsel - 1: test the new neighbour
+    __syncwarp();
+    // against the survivors before it in this tile
+    uint32_t fire = 0, amb = 0;
+    for (uint32_t q0 = 0; q0 + 1 < ns; q0 += kScreenCols) {
+      const bool in = (uint32_t)lane < ns;
+      const uint32_t nb = min(kScreenCols, ns - q0);
+      const uint2 scr = screen_rows<false>(data, dim, rule, in ? k.tid[lane] : kInv,
+                                           in ? k.tnorm[lane] : 0.0f, in ? k.tdis[lane] : 0.0f,
+                                           k.tid + q0, k.tnorm + q0, k.tdis + q0, nb, k.tile);
+      fire |= scr.x << q0;
+      amb |= scr.y << q0;
+      if (in)
+        for (uint32_t q = q0; q < min(q0 + nb, (uint32_t)lane); ++q)
+          if (k.tid[q] == k.tid[lane]) fire |= 1u << q;
     }
-  }
-  __syncwarp();
-  if (scored) *scored = __reduce_add_sync(kFull, rows);
-  if (nsel == fd) return fd - 1;
-  if (nsel >= 2 && last_pos == len - 1) return nsel - 1;
-  return nsel;
-}
-
-// The same filter, warp-cooperative (where wide_filter picks it). A
-// thread-serial distance over a wide row is a long chain of scattered 16-byte
-// loads per lane; here the warp takes the candidates in list order and tests
-// each against the kept neighbours G at a time with coalesced row reads,
-// stopping at the first group in which a rule fires. A candidate is dropped
-// when any of its tests fires, whichever fires first, so the kept set and the
-// return value are those of warp_filter. G kept neighbours per step: 8 at 96 dims (warp_dist8_d96, a half-warp per
-// distance), 4 otherwise (warp_dist4). DIM != 0 fixes the width at compile
-// time. At 128 dims (one chunk per lane) the candidate's chunk is loaded once
-// for all its tests; at 960 the eight chunks a lane would hold cost more in
-// registers than their reloads (NSSG at 1M x 960: 0.80 s against 0.54 s).
-template <int G, uint32_t DIM>
-static __device__ __noinline__ uint32_t warp_filter_group(const uint32_t* cand, const float* cdis,
-                                                          uint32_t len, uint32_t bid, uint32_t fd,
-                                                          int metric, float thre,
-                                                          const __half* __restrict__ data,
-                                                          uint32_t dim, uint32_t* sel, float* seld,
-                                                          int lane, uint32_t* scored) {
-  uint32_t nsel = 0, last_pos = 0, rows = 0;
-  for (uint32_t i = 0; i < len && nsel < fd; ++i) {
-    const uint32_t c = cand[i];
-    if (c == bid || c == kInv) continue;
-    const float dc = cdis[i];
-    const __half* crow = data + (size_t)c * dim;
-    bool keep = true;
-    constexpr bool kPreload = G == 4 && DIM != 0 && DIM <= 128;
-    [[maybe_unused]] QRow<kPreload ? DIM : 4u> qr;
-    if constexpr (kPreload)
-      if (nsel > 0) load_qrow(crow, qr, lane);
-    for (uint32_t s0 = 0; s0 < nsel && keep; s0 += G) {
-      uint32_t ids[G];
-      float o[G];
-#pragma unroll
-      for (int t = 0; t < G; ++t) {
-        ids[t] = s0 + t < nsel ? sel[s0 + t] : kInv;
-        if (ids[t] == c) keep = false;  // a repeat of a kept neighbour (:1423-1427)
+    uint32_t kept = 0;  // survivors kept so far
+    for (uint32_t r = 0; r < ns && nsel < fd; ++r) {
+      if (__shfl_sync(kFull, fire, (int)r) & kept) continue;
+      bool out = false;
+      for (uint32_t m = __shfl_sync(kFull, amb, (int)r) & kept; m && !out; m &= m - 1u) {
+        const uint32_t q = __ffs(m) - 1;
+        out = exact_test(data, dim, rule, k.tid[r], k.tdis[r], k.tid[q], k.tdis[q]);
       }
-      if (!keep) break;
-      if constexpr (G == 8)
-        warp_dist8_d96(crow, data, ids, o, lane);
-      else if constexpr (kPreload)
-        warp_dist4_q<DIM>(qr, data, ids, o, lane);
-      else
-        warp_dist4<DIM>(crow, data, dim, ids, o, lane);
-#pragma unroll
-      for (int t = 0; t < G; ++t) {
-        if (ids[t] == kInv) continue;
-        ++rows;
-        if (pruned_by(metric, o[t], dc, seld[s0 + t], thre)) keep = false;
-      }
-    }
-    if (keep) {
+      if (out) continue;
+      kept |= 1u << r;
       if (lane == 0) {
-        sel[nsel] = c;
-        seld[nsel] = dc;
+        k.id[nsel] = k.tid[r];
+        k.dis[nsel] = k.tdis[r];
+        k.norm[nsel] = k.tnorm[r];
       }
-      __syncwarp();
       ++nsel;
-      last_pos = i;
+      // the r-th survivor's place in the list
+      uint32_t a = alive;
+      for (uint32_t x = 0; x < r; ++x) a &= a - 1u;
+      last = base + __ffs(a) - 1;
     }
+    __syncwarp();
   }
   __syncwarp();
-  if (scored) *scored = rows;
   if (nsel == fd) return fd - 1;
-  if (nsel >= 2 && last_pos == len - 1) return nsel - 1;
+  if (nsel >= 2 && last == len - 1 && tail) return nsel - 1;
   return nsel;
-}
-
-// Which filter a prune runs. Measured at 1M-2M nodes: the cooperative filter
-// wins wherever the thread-serial tree is not the 128-dim one (d = 96: the
-// Vamana select 1,098 -> 466 ms; d = 960: NSSG 5.5 -> 0.51 s) and, at 128
-// dims, where alpha > 1 keeps long lists that take many tests per candidate
-// (Vamana 1.2: 262 -> 170 ms). At 128 dims with alpha 1 most candidates fall
-// to their first tests, and 32 lanes each working through its own candidate
-// keep more loads in flight (NSG select 203 ms against 226).
-__device__ __forceinline__ bool wide_filter(uint32_t dim, int metric, float thre) {
-  return dim != 128 || (metric == 0 && thre > 1.0f);
-}
-
-static __device__ __forceinline__ uint32_t warp_filter_wide(const uint32_t* cand, const float* cdis,
-                                                            uint32_t len, uint32_t bid, uint32_t fd,
-                                                            int metric, float thre,
-                                                            const __half* __restrict__ data,
-                                                            uint32_t dim, uint32_t* sel, float* seld,
-                                                            int lane, uint32_t* scored) {
-  if (dim == 96)
-    return warp_filter_group<8, 96>(cand, cdis, len, bid, fd, metric, thre, data, dim, sel, seld,
-                                    lane, scored);
-  if (dim == 960)
-    return warp_filter_group<4, 960>(cand, cdis, len, bid, fd, metric, thre, data, dim, sel, seld,
-                                     lane, scored);
-  if (dim == 128)
-    return warp_filter_group<4, 128>(cand, cdis, len, bid, fd, metric, thre, data, dim, sel, seld,
-                                     lane, scored);
-  return warp_filter_group<4, 0>(cand, cdis, len, bid, fd, metric, thre, data, dim, sel, seld,
-                                 lane, scored);
 }
 
 // Per-warp shared layout of the select kernels: the beam (path collect) and
 // the candidate list share one region, since the list is filled only after
 // the beam has finished (its ring of scored nodes lives in global memory).
 struct SelLayout {
-  uint32_t W, L, fd;
+  uint32_t W, L;
+  size_t tail;  // bytes behind the list (kept_bytes where the kernel also filters)
   __host__ __device__ size_t bytes() const {
-    const size_t list = (size_t)L * 8 + (size_t)fd * 8;
+    const size_t list = (size_t)L * 8 + tail;
     const size_t beam = W ? beam_bytes(W) : 0;
     return ((beam > list ? beam : list) + 64 + 15) & ~(size_t)15;
   }
@@ -669,9 +630,6 @@ __global__ void k_cal_ep(const uint32_t* __restrict__ G, const __half* __restric
   if (lane == 0) *ep = best;
 }
 
-// select_path (:1498-1517) and select_2hop (:1520-1534) into scratch rows.
-// path: collect_path + Filter_path(distance_filter); 2-hop: collect_2hop +
-// Filter_path(angle_filter). The reference always uses these two filters.
 // Node handed to this warp: one shared counter, taken a node at a time, keeps
 // the SMs busy to the end whatever the per-node search length.
 __device__ __forceinline__ uint32_t next_node(uint32_t* ctr, int lane) {
@@ -684,109 +642,218 @@ __device__ __forceinline__ uint32_t node_at(const uint32_t* __restrict__ order, 
   return order ? __ldg(order + i) : i;
 }
 
-// ring_ids / ring_dis: per-warp rings of kSelectCand scored nodes (path
-// collect), indexed by the warp's global number.
+// The collect half of select_path (:1498-1517) and select_2hop (:1520-1534):
+// node b's sorted candidate list (its kNN row and the collected nodes) without
+// repeats and b itself, in cand / cdis. Returns its length; *scored adds the
+// rows scored. rid / rds: this warp's ring of kSelectCand scored nodes (path).
+template <bool kPath>
+__device__ __forceinline__ uint32_t collect_node(
+    const uint32_t* __restrict__ G, const float* __restrict__ nd, const __half* __restrict__ data,
+    uint32_t dim, uint32_t K, uint32_t ep, uint32_t topm, uint32_t b, Beam bm, uint32_t* rid,
+    float* rds, uint32_t* cand, float* cdis, bool* tail, uint32_t* scored, int lane) {
+  const __half* q = data + (size_t)b * dim;
+  *scored = kSelectCand;  // 2-hop: the 480 collected
+  if (kPath) {
+    uint32_t curr = 0;
+    warp_beam(G, data, dim, K, q, ep, topm, 10, bm, rid, rds, &curr, lane);
+    *scored = curr;
+    __syncwarp();  // the ring (global) and the beam's region are done
+    for (uint32_t i = lane; i < kSelectCand; i += 32) {
+      const bool in = i < curr;
+      cand[K + i] = in ? rid[i] : kInv;
+      cdis[K + i] = in ? rds[i] : kInfDis;
+    }
+  } else {
+    for (uint32_t i = lane; i < kSelectCand; i += 32)
+      cand[K + i] = __ldg(G + (size_t)__ldg(G + (size_t)b * K + i / K) * K + i % K);
+    __syncwarp();
+    // The two-hop rows are scored four at a time by the whole warp: each
+    // lane reads its 8-byte chunks of four rows at once (coalesced across
+    // the warp) and the four shuffle trees interleave. Same lane order as
+    // the thread-serial distance, so the same values.
+    auto score = [&](auto&& dist4) {
+      for (uint32_t i = 0; i < kSelectCand; i += 4) {
+        const uint32_t ids[4] = {cand[K + i], cand[K + i + 1], cand[K + i + 2], cand[K + i + 3]};
+        float o[4];
+        dist4(ids, o);
+        if (lane < 4)
+          cdis[K + i + lane] = lane == 0 ? o[0] : lane == 1 ? o[1] : lane == 2 ? o[2] : o[3];
+      }
+    };
+    if (dim == 960) {
+      score([&](const uint32_t* ids, float* o) { warp_dist4<960>(q, data, dim, ids, o, lane); });
+    } else {
+      score([&](const uint32_t* ids, float* o) { warp_dist4(q, data, dim, ids, o, lane); });
+    }
+  }
+  for (uint32_t i = lane; i < K; i += 32) {
+    cand[i] = __ldg(G + (size_t)b * K + i);
+    cdis[i] = nd[(size_t)b * K + i];
+  }
+  __syncwarp();
+  warp_sort_mark(cand, cdis, kSelectCand + K, lane);
+  return warp_compact(cand, cdis, kSelectCand + K, b, tail, lane);
+}
+
+// The filter half: select_path and select_2hop always use distance_filter and
+// angle_filter respectively. Results go to scratch rows, and the selected
+// distances to the node's own nd row, which no other node reads.
+__device__ __forceinline__ void filter_node(const uint32_t* cand, const float* cdis, uint32_t len,
+                                            bool tail, uint32_t fd, int metric, float thre,
+                                            const __half* __restrict__ data,
+                                            const float* __restrict__ norms, uint32_t dim,
+                                            const Kept& k, uint32_t b, uint32_t K,
+                                            float* __restrict__ nd, uint32_t* __restrict__ P_ids,
+                                            float* __restrict__ P_dis,
+                                            uint32_t* __restrict__ P_cnt, int lane) {
+  const uint32_t stored =
+      warp_filter(cand, cdis, len, tail, fd, metric, thre, data, norms, dim, k, lane);
+  for (uint32_t i = lane; i < stored; i += 32) {
+    P_ids[(size_t)b * fd + i] = k.id[i];
+    P_dis[(size_t)b * fd + i] = k.dis[i];
+    nd[(size_t)b * K + i] = k.dis[i];
+  }
+  if (lane == 0) P_cnt[b] = stored;
+  __syncwarp();
+}
+
+// Candidate lists of the nodes at positions [first, first + cnt) of the order,
+// L entries apart; L_cnt holds a list's length and, in its top bit, `tail`.
+// ring_ids / ring_dis: per-warp rings of kSelectCand scored nodes (path), by the
+// warp's global number.
+//
+// Collect and filter are two kernels with the list between them in memory
+// (about 4 KB written and read per node, 1.4 ms of a 1M prune): the beam waits on
+// gathers and wants warps, the filter's tiles want registers, and each half's
+// code fits the instruction cache.
+constexpr uint32_t kTailBit = 0x80000000u;
+
 template <bool kPath>
 __global__ void __launch_bounds__(kWarps * 32, 6)
-    k_select(const uint32_t* __restrict__ G, float* __restrict__ nd, const __half* __restrict__ data,
-             uint32_t n, uint32_t dim, uint32_t K, const uint32_t* __restrict__ ep_dev,
-             uint32_t* __restrict__ ctr, uint32_t topm, uint32_t fd, float thre,
-             uint32_t* __restrict__ P_ids, float* __restrict__ P_dis, uint32_t* __restrict__ P_cnt,
-             unsigned long long* __restrict__ work, uint32_t* __restrict__ ring_ids,
-             float* __restrict__ ring_dis, const uint32_t* __restrict__ order) {
+    k_collect(const uint32_t* __restrict__ G, const float* __restrict__ nd,
+              const __half* __restrict__ data, uint32_t first, uint32_t cnt, uint32_t dim,
+              uint32_t K, const uint32_t* __restrict__ ep_dev, uint32_t* __restrict__ ctr,
+              uint32_t topm, uint32_t* __restrict__ L_ids, float* __restrict__ L_dis,
+              uint32_t* __restrict__ L_cnt, unsigned long long* __restrict__ work,
+              uint32_t* __restrict__ ring_ids, float* __restrict__ ring_dis,
+              const uint32_t* __restrict__ order) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  SelLayout lay{kPath ? topm + K : 0u, kSelectCand + K, fd};
+  const SelLayout lay{kPath ? topm + K : 0u, kSelectCand + K, 0};
   unsigned char* mine = smem + (size_t)warp * lay.bytes();
   uint32_t* cand = reinterpret_cast<uint32_t*>(mine);
   float* cdis = reinterpret_cast<float*>(cand + lay.L);
-  uint32_t* sel = reinterpret_cast<uint32_t*>(cdis + lay.L);
-  float* seld = reinterpret_cast<float*>(sel + fd);
   Beam bm = beam_carve(mine, lay.W);  // same region as the list, used before it
   const size_t gw = (size_t)blockIdx.x * kWarps + warp;
   uint32_t* rid = kPath ? ring_ids + gw * kSelectCand : nullptr;
   float* rds = kPath ? ring_dis + gw * kSelectCand : nullptr;
-  const uint32_t L = lay.L;
   const uint32_t ep = kPath ? *ep_dev : 0u;
-  for (uint32_t pos = next_node(ctr, lane); pos < n; pos = next_node(ctr, lane)) {
-    const uint32_t b = node_at(order, pos);
-    const __half* q = data + (size_t)b * dim;
-    uint32_t scored = kSelectCand;  // rows scored for this node (2-hop: the 480 collected)
-    if (kPath) {
-      uint32_t curr = 0;
-      warp_beam(G, data, dim, K, q, ep, topm, 10, bm, rid, rds, &curr, lane);
-      scored = curr;
-      __syncwarp();  // the ring (global) and the beam's region are done
-      for (uint32_t i = lane; i < kSelectCand; i += 32) {
-        const bool in = i < curr;
-        cand[K + i] = in ? rid[i] : kInv;
-        cdis[K + i] = in ? rds[i] : kInfDis;
-      }
-    } else {
-      for (uint32_t i = lane; i < kSelectCand; i += 32)
-        cand[K + i] = __ldg(G + (size_t)__ldg(G + (size_t)b * K + i / K) * K + i % K);
-      __syncwarp();
-      // The two-hop rows are scored four at a time by the whole warp: each
-      // lane reads its 8-byte chunks of four rows at once (coalesced across
-      // the warp) and the four shuffle trees interleave. Same lane order as
-      // the thread-serial distance, so the same values.
-      auto score = [&](auto&& dist4) {
-        for (uint32_t i = 0; i < kSelectCand; i += 4) {
-          const uint32_t ids[4] = {cand[K + i], cand[K + i + 1], cand[K + i + 2], cand[K + i + 3]};
-          float o[4];
-          dist4(ids, o);
-          if (lane < 4)
-            cdis[K + i + lane] = lane == 0 ? o[0] : lane == 1 ? o[1] : lane == 2 ? o[2] : o[3];
-        }
-      };
-      if (dim == 960) {
-        score([&](const uint32_t* ids, float* o) { warp_dist4<960>(q, data, dim, ids, o, lane); });
-      } else {
-        score([&](const uint32_t* ids, float* o) { warp_dist4(q, data, dim, ids, o, lane); });
-      }
+  unsigned long long rows = 0;
+  for (uint32_t i = next_node(ctr, lane); i < cnt; i = next_node(ctr, lane)) {
+    const uint32_t b = node_at(order, first + i);
+    bool tail = false;
+    uint32_t scored = 0;
+    const uint32_t len = collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand,
+                                             cdis, &tail, &scored, lane);
+    rows += scored + len;
+    for (uint32_t j = lane; j < len; j += 32) {
+      L_ids[(size_t)i * lay.L + j] = cand[j];
+      L_dis[(size_t)i * lay.L + j] = cdis[j];
     }
-    for (uint32_t i = lane; i < K; i += 32) {
-      cand[i] = __ldg(G + (size_t)b * K + i);
-      cdis[i] = nd[(size_t)b * K + i];
-    }
-    __syncwarp();
-    warp_sort_mark(cand, cdis, L, lane);
-    uint32_t filtered = 0;
-    const uint32_t stored =
-        wide_filter(dim, kPath ? 0 : 1, thre)
-            ? warp_filter_wide(cand, cdis, L, b, fd, kPath ? 0 : 1, thre, data, dim, sel, seld,
-                               lane, &filtered)
-            : warp_filter(cand, cdis, L, b, fd, kPath ? 0 : 1, thre, data, dim, sel, seld, lane,
-                          &filtered);
-    if (work && lane == 0) atomicAdd(work, (unsigned long long)(scored + filtered));
-    for (uint32_t i = lane; i < stored; i += 32) {
-      P_ids[(size_t)b * fd + i] = sel[i];
-      P_dis[(size_t)b * fd + i] = seld[i];
-      nd[(size_t)b * K + i] = seld[i];  // own row only: no other block reads it
-    }
-    if (lane == 0) P_cnt[b] = stored;
+    if (lane == 0) L_cnt[i] = len | (tail ? kTailBit : 0u);
     __syncwarp();
   }
+  if (work && lane == 0) atomicAdd(work, rows);
+}
+
+__global__ void __launch_bounds__(kWarps * 32, 4)
+    k_filter(const uint32_t* __restrict__ L_ids, const float* __restrict__ L_dis,
+             const uint32_t* __restrict__ L_cnt, uint32_t L, float* __restrict__ nd,
+             const __half* __restrict__ data, const float* __restrict__ norms, uint32_t first,
+             uint32_t cnt, uint32_t dim, uint32_t K, uint32_t* __restrict__ ctr, uint32_t fd,
+             int metric, float thre, uint32_t* __restrict__ P_ids, float* __restrict__ P_dis,
+             uint32_t* __restrict__ P_cnt, const uint32_t* __restrict__ order) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Kept k = kept_carve(smem + (size_t)warp * kept_bytes(fd), fd);
+  for (uint32_t i = next_node(ctr, lane); i < cnt; i = next_node(ctr, lane)) {
+    const uint32_t b = node_at(order, first + i), lc = L_cnt[i];
+    filter_node(L_ids + (size_t)i * L, L_dis + (size_t)i * L, lc & ~kTailBit, (lc & kTailBit) != 0,
+                fd, metric, thre, data, norms, dim, k, b, K, nd, P_ids, P_dis, P_cnt, lane);
+  }
+}
+
+// Both halves by the same warp, the list in shared memory: for the prune that
+// may not allocate the lists.
+template <bool kPath>
+__global__ void __launch_bounds__(kWarps * 32, 4)
+    k_select(const uint32_t* __restrict__ G, float* __restrict__ nd, const __half* __restrict__ data,
+             const float* __restrict__ norms, uint32_t n, uint32_t dim, uint32_t K,
+             const uint32_t* __restrict__ ep_dev, uint32_t* __restrict__ ctr, uint32_t topm,
+             uint32_t fd, float thre, uint32_t* __restrict__ P_ids, float* __restrict__ P_dis,
+             uint32_t* __restrict__ P_cnt, uint32_t* __restrict__ ring_ids,
+             float* __restrict__ ring_dis) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const SelLayout lay{kPath ? topm + K : 0u, kSelectCand + K, kept_bytes(fd)};
+  unsigned char* mine = smem + (size_t)warp * lay.bytes();
+  uint32_t* cand = reinterpret_cast<uint32_t*>(mine);
+  float* cdis = reinterpret_cast<float*>(cand + lay.L);
+  const Kept k = kept_carve(reinterpret_cast<unsigned char*>(cdis + lay.L), fd);
+  Beam bm = beam_carve(mine, lay.W);  // same region as the list, used before it
+  const size_t gw = (size_t)blockIdx.x * kWarps + warp;
+  uint32_t* rid = kPath ? ring_ids + gw * kSelectCand : nullptr;
+  float* rds = kPath ? ring_dis + gw * kSelectCand : nullptr;
+  const uint32_t ep = kPath ? *ep_dev : 0u;
+  for (uint32_t b = next_node(ctr, lane); b < n; b = next_node(ctr, lane)) {
+    bool tail = false;
+    uint32_t scored = 0;
+    const uint32_t len = collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand,
+                                             cdis, &tail, &scored, lane);
+    filter_node(cand, cdis, len, tail, fd, kPath ? 0 : 1, thre, data, norms, dim, k, b, K, nd,
+                P_ids, P_dis, P_cnt, lane);
+  }
+}
+
+// Squared norms of the FP16 base for the screens, one warp per row.
+__global__ void k_row_norms(const __half* __restrict__ data, uint32_t n, uint32_t dim,
+                            float* __restrict__ norms) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n;
+       r += (gridDim.x * blockDim.x) >> 5) {
+    const uint2* row = reinterpret_cast<const uint2*>(data + (size_t)r * dim);
+    float x = 0.0f, y = 0.0f;
+    for (uint32_t j = lane; j < dim / 4; j += 32)
+      chunk_acc(__ldg(row + j), make_uint2(0u, 0u), x, y);
+    const float v = warp_tree(x, y);
+    if (lane == 0) norms[r] = v;
+  }
+}
+
+// Shared bytes per warp of k_filter_reverse.
+__host__ __device__ inline size_t reverse_bytes(uint32_t fd, uint32_t K) {
+  return ((size_t)(fd + K) * 8 + kept_bytes(fd) + 15) & ~(size_t)15;
 }
 
 // filter_reverse (:1537-1657) plus the in-place row writes of the select
 // kernels (:1462-1464, :1477): the stored row is the kNN row overwritten by
 // the select result, then by this stage's result.
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(kWarps * 32, 4)
     k_filter_reverse(uint32_t* __restrict__ graph, const float* __restrict__ nd,
                      const uint32_t* __restrict__ rg, const float* __restrict__ rd,
                      const uint32_t* __restrict__ rnum, const __half* __restrict__ data,
-                     uint32_t n, uint32_t dim, uint32_t K, uint32_t fd, int metric, float thre,
+                     const float* __restrict__ norms, uint32_t n, uint32_t dim, uint32_t K,
+                     uint32_t fd, int metric, float thre,
                      const uint32_t* __restrict__ P_ids, const uint32_t* __restrict__ P_cnt,
                      const uint32_t* __restrict__ order) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t cap = fd + K;  // cur_num <= fd - 1, rever_num <= K
-  unsigned char* mine = smem + (size_t)warp * ((size_t)cap * 8 + (size_t)fd * 8 + 16);
+  unsigned char* mine = smem + (size_t)warp * reverse_bytes(fd, K);
   uint32_t* cand = reinterpret_cast<uint32_t*>(mine);
   float* cdis = reinterpret_cast<float*>(cand + cap);
-  uint32_t* sel = reinterpret_cast<uint32_t*>(cdis + cap);
-  float* seld = reinterpret_cast<float*>(sel + fd);
+  const Kept k = kept_carve(reinterpret_cast<unsigned char*>(cdis + cap), fd);
+  uint32_t* sel = k.id;
   for (uint32_t pos = blockIdx.x * kWarps + warp; pos < n; pos += gridDim.x * kWarps) {
     const uint32_t b = node_at(order, pos);
     const uint32_t cur_num = P_cnt[b];
@@ -805,10 +872,9 @@ __global__ void __launch_bounds__(kWarps * 32)
     uint32_t out_cnt;
     if (len > fd) {
       warp_sort_mark(cand, cdis, len, lane);
-      out_cnt = wide_filter(dim, metric, thre)
-                    ? warp_filter_wide(cand, cdis, len, b, fd, metric, thre, data, dim, sel, seld,
-                                       lane, nullptr)
-                    : warp_filter(cand, cdis, len, b, fd, metric, thre, data, dim, sel, seld, lane);
+      bool tail = false;
+      const uint32_t left = warp_compact(cand, cdis, len, b, &tail, lane);
+      out_cnt = warp_filter(cand, cdis, left, tail, fd, metric, thre, data, norms, dim, k, lane);
     } else {
       // Union in ascending reverse-slot order (:1632-1647).
       for (uint32_t i = lane; i < cur_num; i += 32) sel[i] = cand[i];
@@ -842,6 +908,22 @@ __global__ void __launch_bounds__(kWarps * 32)
 }
 
 // ---------------------------------------------------------------------------
+// Orders a node's ids by (detours << 8 | position) ranks with the reference's
+// network and stores the first d.
+__device__ __forceinline__ void rank_store(uint32_t* rank, const uint32_t* nei0, uint32_t K,
+                                           uint32_t d, uint32_t b, uint32_t* __restrict__ hybrid,
+                                           uint32_t* __restrict__ E_tgt,
+                                           uint32_t* __restrict__ E_val, int lane) {
+  warp_network(K, lane, [&](uint32_t u, uint32_t v) { return (rank[u] >> 8) > (rank[v] >> 8); },
+               [&](uint32_t u, uint32_t v) { swap_(rank[u], rank[v]); });
+  for (uint32_t i = lane; i < d; i += 32) {
+    const uint32_t id = nei0[rank[i] & 0xFFu];
+    E_tgt[(size_t)b * d + i] = id;
+    E_val[(size_t)b * d + i] = rank[i] >> 8;
+    hybrid[(size_t)b * K + i] = id;
+  }
+}
+
 // Rank-based prunes. collect_1hop + filter_cagra (:1660-1710): detour[m]
 // counts the kept-earlier neighbours a whose own list holds n_m, over the
 // pairs the reference visits (a in {i, K-1-i : i < K/2}, m > a).
@@ -924,142 +1006,73 @@ __global__ void __launch_bounds__(kWarps * 32)
       rank[m] = (det << 8) | m;
     }
     __syncwarp();
-    warp_network(K, lane, [&](uint32_t u, uint32_t v) { return (rank[u] >> 8) > (rank[v] >> 8); },
-                 [&](uint32_t u, uint32_t v) { swap_(rank[u], rank[v]); });
-    for (uint32_t i = lane; i < d; i += 32) {
-      const uint32_t id = nei0[rank[i] & 0xFFu];
-      E_tgt[(size_t)b * d + i] = id;
-      E_val[(size_t)b * d + i] = rank[i] >> 8;
-      hybrid[(size_t)b * K + i] = id;
-    }
+    rank_store(rank, nei0, K, d, b, hybrid, E_tgt, E_val, lane);
     __syncwarp();
   }
 }
 
 // collect_1hop + filter_dpg (:1713-1785): detour[m] counts earlier a with
-// d(n_a, n_m) < d(u, n_m), each warp using its own vector (see header note).
-__global__ void __launch_bounds__(kWarps * 32)
+// d(n_a, n_m) < d(u, n_m), over the reference's pair set (all a < m but the
+// middle row of an odd K, :1715-1717), each warp using its own vector (see
+// header note). The pairs are screened 32 positions against 16 earlier ones at a
+// time; the few ambiguous ones take the exact distance.
+//
+// Bound by the row gathers, mostly from L1.
+__host__ __device__ inline uint32_t dpg_words(uint32_t K) { return 4 * K + kScreenFloats; }
+
+__global__ void __launch_bounds__(kWarps * 32, 4)
     k_select_dpg(const uint32_t* __restrict__ G, const float* __restrict__ nd,
-                 const __half* __restrict__ data, uint32_t n, uint32_t dim, uint32_t K, uint32_t d,
-                 uint32_t* __restrict__ hybrid, uint32_t* __restrict__ E_tgt,
-                 uint32_t* __restrict__ E_val, const uint32_t* __restrict__ order) {
+                 const __half* __restrict__ data, const float* __restrict__ norms, uint32_t n,
+                 uint32_t dim, uint32_t K, uint32_t d, uint32_t* __restrict__ hybrid,
+                 uint32_t* __restrict__ E_tgt, uint32_t* __restrict__ E_val,
+                 const uint32_t* __restrict__ order) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned char* mine = smem + (size_t)warp * ((size_t)K * 12);
-  uint32_t* nei0 = reinterpret_cast<uint32_t*>(mine);
-  uint32_t* det = nei0 + K;
-  float* nrow = reinterpret_cast<float*>(det + K);
+  uint32_t* nei0 = reinterpret_cast<uint32_t*>(smem) + (size_t)warp * dpg_words(K);
+  float* nrow = reinterpret_cast<float*>(nei0 + K);
+  float* nn = nrow + K;
+  uint32_t* rank = reinterpret_cast<uint32_t*>(nn + K);
+  float* tile = reinterpret_cast<float*>(rank + K);
+  const ScreenRule rule{0, 1.0f, screen_eps(dim)};  // res < d(u, n_m)
   for (uint32_t pos = blockIdx.x * kWarps + warp; pos < n; pos += gridDim.x * kWarps) {
     const uint32_t b = node_at(order, pos);
     for (uint32_t j = lane; j < K; j += 32) {
-      nei0[j] = __ldg(G + (size_t)b * K + j);
-      det[j] = 0;
+      const uint32_t id = __ldg(G + (size_t)b * K + j);
+      nei0[j] = id;
       nrow[j] = nd[(size_t)b * K + j];
+      nn[j] = __ldg(norms + id);
     }
     __syncwarp();
-    for (uint32_t i = 0; i < K / 2; ++i) {
-      for (int side = 0; side < 2; ++side) {
-        const uint32_t a = side ? (K - 1 - i) : i;
-        const uint32_t m0 = side ? (K - i) : (i + 1);
-        const __half* qa = data + (size_t)nei0[a] * dim;
-        for (uint32_t m = m0; m < K; m += 4) {
-          uint32_t ids[4];
-          float r4[4];
-#pragma unroll
-          for (int t = 0; t < 4; ++t) ids[t] = (m + t < K) ? nei0[m + t] : kInv;
-          warp_dist4(qa, data, dim, ids, r4, lane);
-          if (lane == 0) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-              if (m + t < K && r4[t] < nrow[m + t]) det[m + t] += 1;
+    for (uint32_t m0 = 0; m0 < K; m0 += 32) {
+      const uint32_t m = m0 + lane;
+      const uint32_t id = m < K ? nei0[m] : kInv;
+      const float dm = m < K ? nrow[m] : 0.0f, nm = m < K ? nn[m] : 0.0f;
+      uint32_t det = 0;
+      for (uint32_t a0 = 0; a0 < min(m0 + 32, K); a0 += kScreenCols) {
+        const uint2 scr = screen_rows<false>(data, dim, rule, id, nm, dm, nei0 + a0, nn + a0,
+                                             nrow + a0, min(kScreenCols, K - a0), tile);
+        // a < m, and not the middle row of an odd K
+        uint32_t pairs = m > a0 ? (m - a0 >= 32 ? kFull : (1u << (m - a0)) - 1u) : 0u;
+        if ((K & 1u) && K / 2 >= a0 && K / 2 < a0 + kScreenCols) pairs &= ~(1u << (K / 2 - a0));
+        det += (uint32_t)__popc(scr.x & pairs);
+        uint32_t amb = scr.y & pairs;
+        for (unsigned left = __ballot_sync(kFull, amb != 0); left;
+             left = __ballot_sync(kFull, amb != 0)) {
+          const int o = __ffs(left) - 1;
+          const uint32_t a = a0 + __ffs(__shfl_sync(kFull, amb, o)) - 1;
+          const float res = warp_dist(data + (size_t)nei0[a] * dim,
+                                      data + (size_t)__shfl_sync(kFull, id, o) * dim, dim, lane);
+          if (lane == o) {
+            det += res < dm ? 1u : 0u;
+            amb &= amb - 1u;
           }
-          __syncwarp();
         }
       }
-    }
-    warp_network(K, lane, [&](uint32_t u, uint32_t v) { return det[u] > det[v]; },
-                 [&](uint32_t u, uint32_t v) {
-                   swap_(det[u], det[v]);
-                   swap_(nei0[u], nei0[v]);
-                 });
-    for (uint32_t i = lane; i < d; i += 32) {
-      E_tgt[(size_t)b * d + i] = nei0[i];
-      E_val[(size_t)b * d + i] = det[i];
-      hybrid[(size_t)b * K + i] = nei0[i];
+      if (m < K) rank[m] = (det << 8) | m;
     }
     __syncwarp();
-  }
-}
-
-// The same select for wide rows, one node per block. The node's K neighbour
-// rows (123 KB at K = 64, d = 960) are read by all K(K-1)/2 pair distances;
-// with one 1,024-thread block per SM they stay in that SM's L1 while its 32
-// warps share the pairs. Work items are (a, m0): row a against the four rows
-// m0..m0+3 (m > a), over the reference's pair set (a < K/2 from the front,
-// a >= K - K/2 from the back, :1715-1717); detour counts are shared-memory
-// integer atomics, so the order of the items changes no count.
-constexpr int kDpgThreads = 1024;
-
-__global__ void __launch_bounds__(kDpgThreads, 1)
-    k_select_dpg_block(const uint32_t* __restrict__ G, const float* __restrict__ nd,
-                       const __half* __restrict__ data, uint32_t n, uint32_t dim, uint32_t K,
-                       uint32_t d, uint32_t* __restrict__ hybrid, uint32_t* __restrict__ E_tgt,
-                       uint32_t* __restrict__ E_val, const uint32_t* __restrict__ order) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kBlockWarps = kDpgThreads / 32;
-  uint32_t* nei0 = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* det = nei0 + K;
-  float* nrow = reinterpret_cast<float*>(det + K);
-  uint16_t* items = reinterpret_cast<uint16_t*>(nrow + K);  // (a << 8) | m0
-  __shared__ uint32_t n_items;
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (uint32_t a = 0; a + 1 < K; ++a) {
-      if (a >= K / 2 && a < K - K / 2) continue;  // the middle row of an odd K (:1715-1717)
-      for (uint32_t m0 = a + 1; m0 < K; m0 += 4) items[t++] = (uint16_t)((a << 8) | m0);
-    }
-    n_items = t;
-  }
-  __syncthreads();
-  const uint32_t T = n_items;
-  for (uint32_t pos = blockIdx.x; pos < n; pos += gridDim.x) {
-    const uint32_t b = node_at(order, pos);
-    for (uint32_t j = threadIdx.x; j < K; j += kDpgThreads) {
-      nei0[j] = __ldg(G + (size_t)b * K + j);
-      det[j] = 0;
-      nrow[j] = nd[(size_t)b * K + j];
-    }
-    __syncthreads();
-    for (uint32_t t = warp; t < T; t += kBlockWarps) {
-      const uint32_t a = items[t] >> 8, m0 = items[t] & 0xFFu;
-      uint32_t ids[4];
-      float r4[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) ids[q] = (m0 + q < K) ? nei0[m0 + q] : kInv;
-      if (dim == 960)
-        warp_dist4<960>(data + (size_t)nei0[a] * dim, data, dim, ids, r4, lane);
-      else
-        warp_dist4(data + (size_t)nei0[a] * dim, data, dim, ids, r4, lane);
-      if (lane < 4 && m0 + lane < K) {
-        const float r = lane == 0 ? r4[0] : lane == 1 ? r4[1] : lane == 2 ? r4[2] : r4[3];
-        if (r < nrow[m0 + lane]) atomicAdd(&det[m0 + lane], 1u);
-      }
-    }
-    __syncthreads();
-    if (warp == 0) {
-      warp_network(K, lane, [&](uint32_t u, uint32_t v) { return det[u] > det[v]; },
-                   [&](uint32_t u, uint32_t v) {
-                     swap_(det[u], det[v]);
-                     swap_(nei0[u], nei0[v]);
-                   });
-      for (uint32_t i = lane; i < d; i += 32) {
-        E_tgt[(size_t)b * d + i] = nei0[i];
-        E_val[(size_t)b * d + i] = det[i];
-        hybrid[(size_t)b * K + i] = nei0[i];
-      }
-    }
-    __syncthreads();
+    rank_store(rank, nei0, K, d, b, hybrid, E_tgt, E_val, lane);
+    __syncwarp();
   }
 }
 
@@ -1302,7 +1315,6 @@ int set_smem(const void* fn, size_t bytes) {
   return TAGORE_OK;
 }
 
-// Select (path or 2-hop) + reverse store + filter_reverse.
 // The select's processing order (see k_label_min), in scratch `sc`.
 int locality_order(const Dev& d, Scratch& sc, const uint32_t** order, cudaStream_t s) {
   const uint32_t n = d.n, hops = std::min(kLabelHops, d.k);
@@ -1331,19 +1343,55 @@ int locality_order(const Dev& d, Scratch& sc, const uint32_t** order, cudaStream
   return TAGORE_OK;
 }
 
+int reverse_grid(uint32_t fd, uint32_t K, uint32_t n, int* grid) {
+  const size_t sm = reverse_bytes(fd, K) * kWarps;
+  TG_TRY(set_smem((const void*)k_filter_reverse, sm));
+  return resident_grid((const void*)k_filter_reverse, kWarps * 32, sm, kWarps, n, grid);
+}
+
+// Nodes per collect / filter pair: bounds the candidate lists in memory (about
+// 1.2 GB at K = 96) and still fills the chip hundreds of times over.
+constexpr uint32_t kSelectBatch = 1u << 18;
+
+void launch_row_norms(const Dev& d, float* norms, cudaStream_t s) {
+  k_row_norms<<<grid_for(8, d.n), 256, 0, s>>>(d.data, d.n, d.dim, norms);
+  count_launch();
+}
+
+int launch_filter_reverse(const Dev& d, int grid, const float* norms, uint32_t fd, int metric,
+                          float thre, const uint32_t* P_ids, const uint32_t* P_cnt,
+                          const uint32_t* order, cudaStream_t s) {
+  const size_t sm = reverse_bytes(fd, d.k) * kWarps;
+  TG_TRY(set_smem((const void*)k_filter_reverse, sm));
+  k_filter_reverse<<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.rgraph, d.rd, d.rnum, d.data,
+                                                 norms, d.n, d.dim, d.k, fd, metric, thre, P_ids,
+                                                 P_cnt, order);
+  count_launch();
+  TG_CUDA(cudaGetLastError());
+  return TAGORE_OK;
+}
+
+// Collect (path or 2-hop) and filter, then reverse store and filter_reverse.
 int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint32_t* ep_host,
                    cudaStream_t s) {
   const uint32_t fd = a.final_degree, K = d.k;
   if (!path && K * K < kSelectCand) return fail(TAGORE_EINVAL, "2-hop collect needs K*K >= 480");
   if (path && (a.topm == 0 || a.topm > 256)) return fail(TAGORE_EINVAL, "TOPM must be in [1, 256]");
+  const SelLayout lay{path ? a.topm + K : 0u, kSelectCand + K, 0};
+  const uint32_t batch = std::min(d.n, kSelectBatch), batches = (d.n + batch - 1) / batch;
   Scratch sc(s);
-  TG_TRY(sc.alloc(16 + (size_t)d.n * fd * 8 + (size_t)d.n * 4));
-  // [u64 rows scored][u32 entry point][u32 node counter] | select rows
+  // [u64 rows scored][u32 entry point][u32 unused][2 u32 counters per batch] |
+  // select rows | norms
+  const size_t head = 16 + (((size_t)batches * 8 + 15) & ~(size_t)15);
+  TG_TRY(sc.alloc(head + (size_t)d.n * fd * 8 + (size_t)d.n * 8));
   unsigned long long* work = sc.as<unsigned long long>();
   uint32_t* ep_dev = reinterpret_cast<uint32_t*>(work + 1);
-  uint32_t* P_ids = ep_dev + 2;
+  uint32_t* ctr = ep_dev + 2;
+  uint32_t* P_ids = reinterpret_cast<uint32_t*>(sc.as<unsigned char>() + head);
   float* P_dis = reinterpret_cast<float*>(P_ids + (size_t)d.n * fd);
   uint32_t* P_cnt = reinterpret_cast<uint32_t*>(P_dis + (size_t)d.n * fd);
+  float* norms = reinterpret_cast<float*>(P_cnt + d.n);
+  TG_CUDA(cudaMemsetAsync(work, 0, head, s));
   if (path) {
     const uint32_t W = a.topm + K;
     const size_t sm = beam_bytes(W) + 64;
@@ -1354,58 +1402,68 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
     stage_end("prune_cal_ep", s);
     TG_CUDA(cudaGetLastError());
   }
-  SelLayout lay{path ? a.topm + K : 0u, kSelectCand + K, fd};
-  const size_t sm = lay.bytes() * kWarps;
-  const void* fn = path ? (const void*)k_select<true> : (const void*)k_select<false>;
+  const size_t sm = lay.bytes() * kWarps, smf = kept_bytes(fd) * kWarps;
+  const void* fn = path ? (const void*)k_collect<true> : (const void*)k_collect<false>;
   TG_TRY(set_smem(fn, sm));
-  int grid = 0;
-  TG_TRY(resident_grid(fn, kWarps * 32, sm, kWarps, d.n, &grid));
-  Scratch rings(s);
+  TG_TRY(set_smem((const void*)k_filter, smf));
+  int grid = 0, gridf = 0;
+  TG_TRY(resident_grid(fn, kWarps * 32, sm, kWarps, batch, &grid));
+  TG_TRY(resident_grid((const void*)k_filter, kWarps * 32, smf, kWarps, batch, &gridf));
+  Scratch rings(s), lists(s);
   if (path) TG_TRY(rings.alloc((size_t)grid * kWarps * kSelectCand * 8));
   uint32_t* ring_ids = path ? rings.as<uint32_t>() : nullptr;
   float* ring_dis =
       path ? reinterpret_cast<float*>(ring_ids + (size_t)grid * kWarps * kSelectCand) : nullptr;
-  uint32_t* ctr = ep_dev + 1;
-  TG_CUDA(cudaMemsetAsync(work, 0, 8, s));
-  TG_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t), s));
+  TG_TRY(lists.alloc((size_t)batch * (lay.L * 8 + 4)));
+  uint32_t* L_ids = lists.as<uint32_t>();
+  float* L_dis = reinterpret_cast<float*>(L_ids + (size_t)batch * lay.L);
+  uint32_t* L_cnt = reinterpret_cast<uint32_t*>(L_dis + (size_t)batch * lay.L);
   Scratch ord(s);
   const uint32_t* order = nullptr;
   stage_begin("prune_order", s);
   TG_TRY(locality_order(d, ord, &order, s));
+  launch_row_norms(d, norms, s);
   stage_end("prune_order", s);
   const char* sel_name = path ? "prune_select_path" : "prune_select_2hop";
-  stage_begin(sel_name, s);
-  if (path)
-    k_select<true><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, d.n, d.dim, K, ep_dev, ctr,
-                                                 a.topm, fd, a.thre, P_ids, P_dis, P_cnt, work,
-                                                 ring_ids, ring_dis, order);
-  else
-    k_select<false><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, d.n, d.dim, K, ep_dev,
-                                                  ctr, a.topm, fd, a.thre, P_ids, P_dis, P_cnt,
-                                                  work, nullptr, nullptr, order);
-  count_launch();
-  stage_end(sel_name, s);
-  TG_CUDA(cudaGetLastError());
+  for (uint32_t i = 0; i < batches; ++i) {
+    const uint32_t first = i * batch, cnt = std::min(batch, d.n - first);
+    stage_begin(sel_name, s);
+    if (path)
+      k_collect<true><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, first, cnt, d.dim, K,
+                                                    ep_dev, ctr + 2 * i, a.topm, L_ids, L_dis,
+                                                    L_cnt, work, ring_ids, ring_dis, order);
+    else
+      k_collect<false><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, first, cnt, d.dim, K,
+                                                     ep_dev, ctr + 2 * i, a.topm, L_ids, L_dis,
+                                                     L_cnt, work, nullptr, nullptr, order);
+    count_launch();
+    stage_end(sel_name, s);
+    TG_CUDA(cudaGetLastError());
+    stage_begin("prune_filter", s);
+    k_filter<<<gridf, kWarps * 32, smf, s>>>(L_ids, L_dis, L_cnt, lay.L, d.nd, d.data, norms, first,
+                                             cnt, d.dim, K, ctr + 2 * i + 1, fd, path ? 0 : 1,
+                                             a.thre, P_ids, P_dis, P_cnt, order);
+    count_launch();
+    stage_end("prune_filter", s);
+    TG_CUDA(cudaGetLastError());
+  }
   stage_begin("prune_reverse_store", s);
   TG_TRY(reverse_store(d, P_ids, reinterpret_cast<const uint32_t*>(P_dis), P_cnt, fd, 0, K, K, s));
   stage_end("prune_reverse_store", s);
-  const size_t sm2 = ((size_t)(fd + K) * 8 + (size_t)fd * 8 + 16) * kWarps;
-  TG_TRY(set_smem((const void*)k_filter_reverse, sm2));
+  int gridr = 0;
+  TG_TRY(reverse_grid(fd, K, d.n, &gridr));
   stage_begin("prune_filter_reverse", s);
-  k_filter_reverse<<<grid, kWarps * 32, sm2, s>>>(d.graph, d.nd, d.rgraph, d.rd, d.rnum, d.data,
-                                                  d.n, d.dim, K, fd, metric, a.thre, P_ids, P_cnt,
-                                                  order);
-  count_launch();
+  TG_TRY(launch_filter_reverse(d, gridr, norms, fd, metric, a.thre, P_ids, P_cnt, order, s));
   stage_end("prune_filter_reverse", s);
-  TG_CUDA(cudaGetLastError());
   if (path && ep_host) {
     TG_CUDA(cudaMemcpyAsync(ep_host, ep_dev, 4, cudaMemcpyDeviceToHost, s));
   }
   unsigned long long rows = 0;
   if (profiling()) TG_CUDA(cudaMemcpyAsync(&rows, work, 8, cudaMemcpyDeviceToHost, s));
   TG_CUDA(cudaStreamSynchronize(s));
-  // select traffic: every scored row (2d bytes), the kNN row and distances
-  // read (8 B per slot), the selected ids and distances written (8 B each)
+  // select traffic: every scored row and every listed candidate's row (2d
+  // bytes), the kNN row and distances read (8 B per slot), the selected ids and
+  // distances written (8 B each)
   if (profiling())
     stage_add(sel_name, rows * 2ull * d.dim + (uint64_t)d.n * (8ull * K + 8ull * fd + 4), d.n);
   return TAGORE_OK;
@@ -1422,9 +1480,10 @@ int run_rank_prune(const Dev& d, const PruneArgs& a, bool dpg, cudaStream_t s) {
     cap = K - dd - 1;
   }
   Scratch sc(s);
-  TG_TRY(sc.alloc((size_t)d.n * dd * 8 + 16));
+  TG_TRY(sc.alloc((size_t)d.n * dd * 8 + (dpg ? (size_t)d.n * 4 : 0) + 16));
   uint32_t* E_tgt = sc.as<uint32_t>();
   uint32_t* E_val = E_tgt + (size_t)d.n * dd;
+  float* norms = reinterpret_cast<float*>(E_val + (size_t)d.n * dd);  // DPG only
   const int grid = grid_for(kWarps, d.n);
   Scratch ord(s);
   const uint32_t* order = nullptr;
@@ -1438,21 +1497,12 @@ int run_rank_prune(const Dev& d, const PruneArgs& a, bool dpg, cudaStream_t s) {
     TG_TRY(set_smem((const void*)k_select_cagra, sm));
     k_select_cagra<<<grid, kWarps * 32, sm, s>>>(d.graph, d.n, K, dd, d.hybrid, E_tgt, E_val,
                                                  order);
-  } else if (d.dim > 128 && K <= 128) {
-    // the three K-arrays, then the (a, m0) items: fewer than (K/2 + 1)(K/4 + 2) * 2
-    const size_t sm = (size_t)K * 12 + (size_t)(K / 2 + 1) * ((K + 3) / 4 + 1) * 2 * 2 + 16;
-    TG_TRY(set_smem((const void*)k_select_dpg_block, sm));
-    int dev = 0, sms = 148;
-    TG_CUDA(cudaGetDevice(&dev));
-    TG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int g = (int)std::min<uint64_t>(d.n, (uint64_t)sms);
-    k_select_dpg_block<<<g, kDpgThreads, sm, s>>>(d.graph, d.nd, d.data, d.n, d.dim, K, dd,
-                                                  d.hybrid, E_tgt, E_val, order);
   } else {
-    const size_t sm = ((size_t)K * 12) * kWarps;
+    launch_row_norms(d, norms, s);
+    const size_t sm = (size_t)dpg_words(K) * 4 * kWarps;
     TG_TRY(set_smem((const void*)k_select_dpg, sm));
-    k_select_dpg<<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, d.n, d.dim, K, dd, d.hybrid,
-                                               E_tgt, E_val, order);
+    k_select_dpg<<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, norms, d.n, d.dim, K, dd,
+                                               d.hybrid, E_tgt, E_val, order);
   }
   count_launch();
   TG_CUDA(cudaGetLastError());
@@ -1553,7 +1603,7 @@ int prune_cfs_static(const Dev& d, const PruneArgs& a, const std::string& mode,
   const size_t tmp = std::max(sort_tmp, scan_tmp);
   // The select kernel's grid is capped here so that its per-warp rings of
   // scored nodes (path collect) stay small: 64 blocks, under 1 MB.
-  SelLayout lay{path ? a.topm + K : 0u, kSelectCand + K, fd};
+  SelLayout lay{path ? a.topm + K : 0u, kSelectCand + K, kept_bytes(fd)};
   const size_t sm = lay.bytes() * kWarps;
   const void* fn = path ? (const void*)k_select<true> : (const void*)k_select<false>;
   TG_TRY(set_smem(fn, sm));
@@ -1625,14 +1675,19 @@ int prune_cfs_static(const Dev& d, const PruneArgs& a, const std::string& mode,
     count_launch();
     TG_CUDA(cudaGetLastError());
   }
+  // The screens' norms take the place of the reverse-edge keys (E >= n words),
+  // which are written after the select and read before filter_reverse.
+  float* norms = reinterpret_cast<float*>(keys);
+  launch_row_norms(d, norms, s);
+  TG_CUDA(cudaGetLastError());
   if (path)
-    k_select<true><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, d.n, d.dim, K, ep_dev, ctr,
-                                                 a.topm, fd, a.thre, P_ids, P_dis, P_cnt, nullptr,
-                                                 ring_ids, ring_dis, nullptr);
+    k_select<true><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, norms, d.n, d.dim, K,
+                                                 ep_dev, ctr, a.topm, fd, a.thre, P_ids, P_dis,
+                                                 P_cnt, ring_ids, ring_dis);
   else
-    k_select<false><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, d.n, d.dim, K, ep_dev,
-                                                  ctr, a.topm, fd, a.thre, P_ids, P_dis, P_cnt,
-                                                  nullptr, nullptr, nullptr, nullptr);
+    k_select<false><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, norms, d.n, d.dim, K,
+                                                  ep_dev, ctr, a.topm, fd, a.thre, P_ids, P_dis,
+                                                  P_cnt, nullptr, nullptr);
   count_launch();
   TG_CUDA(cudaGetLastError());
 
@@ -1653,13 +1708,8 @@ int prune_cfs_static(const Dev& d, const PruneArgs& a, const std::string& mode,
   TG_CUDA(cudaGetLastError());
 
   // filter_reverse
-  const size_t sm2 = ((size_t)(fd + K) * 8 + (size_t)fd * 8 + 16) * kWarps;
-  TG_TRY(set_smem((const void*)k_filter_reverse, sm2));
-  k_filter_reverse<<<grid, kWarps * 32, sm2, s>>>(d.graph, d.nd, d.rgraph, d.rd, d.rnum, d.data,
-                                                  d.n, d.dim, K, fd, m, a.thre, P_ids, P_cnt,
-                                                  nullptr);
-  count_launch();
-  TG_CUDA(cudaGetLastError());
+  launch_row_norms(d, norms, s);
+  TG_TRY(launch_filter_reverse(d, grid, norms, fd, m, a.thre, P_ids, P_cnt, nullptr, s));
   if (path && ep_host) TG_CUDA(cudaMemcpyAsync(ep_host, ep_dev, 4, cudaMemcpyDeviceToHost, s));
   TG_CUDA(cudaStreamSynchronize(s));
   return TAGORE_OK;

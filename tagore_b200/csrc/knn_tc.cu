@@ -36,11 +36,18 @@ constexpr int kThreads = kConsumers + 32;    // warp 4: the producer
 constexpr int kStages = 2;                   // row tiles in flight
 constexpr uint32_t kTmemCols = 128;          // one 128-column accumulator
 constexpr uint64_t kWaitNs = 2000000000ull;  // 2 s per wait
-constexpr uint32_t kDone = 0xFFFFFFFFu;      // stage node: the producer has finished
 constexpr float kOneMinusEps = 1.0f - 0.000244140625f;  // 1 - 2^-12, the screen's margin
 
 struct __align__(1024) Tile {
   uint8_t x[2][kMaxList][128];  // [64-half column block][row][128 B], SW128
+};
+
+// What a tile holds: one node, or two whose lists have at most 64 rows each, the
+// second one's from row 64 on. Per half of the tile: the rows and columns of its
+// node are [32 first, total), the new ones [32 first, fresh).
+struct NodeSlot {
+  uint32_t live;  // 0: no more nodes
+  uint32_t first[2], fresh[2], total[2];
 };
 
 struct __align__(1024) TcSmem {
@@ -54,7 +61,7 @@ struct __align__(1024) TcSmem {
   unsigned long long empty_bar[kStages];  // consumers done with the stage
   unsigned long long mma_bar[2];          // accumulator written
   uint32_t taddr;
-  uint32_t node[kStages], nn[kStages], total[kStages];
+  NodeSlot slot[kStages];
   uint32_t filled, consumed;  // producer fills with rows; fills the consumers saw land
   int flag;
 };
@@ -164,11 +171,12 @@ __device__ __forceinline__ float key_max(float a, float b) {
 // 40.7 -> 33.6 ms; 250K x 960: 184.9 -> 178.2 ms.
 template <int T>
 __device__ __forceinline__ void screen_row(uint32_t tmem, const float* __restrict__ h, float hr,
-                                           float kth, uint32_t r, uint32_t nn, uint32_t total,
+                                           float kth, uint32_t r, const NodeSlot& slot,
                                            uint32_t (&bc)[4]) {
-  const uint32_t lane = r & 31u, warp = r >> 5;
-  // columns a row may pair with: all others if r is new, new ones if old; the
-  // warp reads only the column blocks one of its rows needs
+  const uint32_t lane = r & 31u, warp = r >> 5, half = warp >> 1;
+  const uint32_t first = slot.first[half], nn = slot.fresh[half], total = slot.total[half];
+  // columns a row may pair with: all others of its node if r is new, new ones if
+  // old; the warp reads only the column blocks one of its rows needs
   const uint32_t cmax = r < total ? (r < nn ? total : nn) : 0u;
   const uint32_t wmax = __reduce_max_sync(kFull, cmax);
   const bool has_old = warp * 32 + 31 >= nn;
@@ -184,7 +192,7 @@ __device__ __forceinline__ void screen_row(uint32_t tmem, const float* __restric
     }
   };
 #pragma unroll 1
-  for (uint32_t q = 0; q * 32 < wmax; ++q) {
+  for (uint32_t q = first; q * 32 < wmax; ++q) {
     float g[32];
     tmem_ld32(tmem + ((warp * 32u) << 16) + q * 32u, g);
     const float4* h4 = reinterpret_cast<const float4*>(h + q * 32);
@@ -227,12 +235,12 @@ __device__ __forceinline__ void screen_row(uint32_t tmem, const float* __restric
 }
 
 __device__ __forceinline__ void screen_rows(uint32_t T, uint32_t tmem, const float* h, float hr,
-                                            float kth, uint32_t r, uint32_t nn, uint32_t total,
+                                            float kth, uint32_t r, const NodeSlot& slot,
                                             uint32_t (&bc)[4]) {
-  if (T == 2) screen_row<2>(tmem, h, hr, kth, r, nn, total, bc);
-  else if (T == 3) screen_row<3>(tmem, h, hr, kth, r, nn, total, bc);
-  else if (T == 1) screen_row<1>(tmem, h, hr, kth, r, nn, total, bc);
-  else screen_row<4>(tmem, h, hr, kth, r, nn, total, bc);
+  if (T == 2) screen_row<2>(tmem, h, hr, kth, r, slot, bc);
+  else if (T == 3) screen_row<3>(tmem, h, hr, kth, r, slot, bc);
+  else if (T == 1) screen_row<1>(tmem, h, hr, kth, r, slot, bc);
+  else screen_row<4>(tmem, h, hr, kth, r, slot, bc);
 }
 
 // Chunks 2p and 2p+1 of row r (one 16-byte unit of the swizzled tile).
@@ -277,10 +285,107 @@ __device__ __forceinline__ bool consumers_any(bool v) {
   return out != 0;
 }
 
-// Producer warp: walks this block's nodes (blockIdx.x, +gridDim.x, ...),
-// skips those without a join, and fills stage j % kStages with node j: ids,
-// norms and k-th distances (one packed record per row) by the lanes, rows by TMA tile::gather4. Runs
-// kStages nodes ahead of the consumers; ends by publishing kDone.
+// The nodes of a block (positions blockIdx.x, +gridDim.x, ... of the order), 32 at
+// a time, one per lane; those without a join are left out.
+struct NodeWindow {
+  uint32_t next, node = 0;
+  uint2 cnt = {0, 0};
+  unsigned rest = 0, small = 0;  // lanes not taken yet; those of at most 64 rows
+};
+struct NodePair {
+  uint32_t u[2], nn[2], tot[2];  // tot[1] 0: one node
+};
+
+// Takes the next node, and with it the next small one of the window if both have at
+// most 64 rows. False when no node is left. A tile costs its barriers, waits and
+// MMA whether 40 rows are in it or 128, and from the fifth iteration on most lists
+// have fewer than 64.
+// 1M x 128, K = 64, 10 iterations: the joins 135 -> 83 ms, the build 178 -> 128 ms;
+// 165K x 96, 16 iterations: the build 33.6 -> 24.3 ms; 250K x 960: 178 -> 156 ms.
+__device__ __forceinline__ bool take_nodes(NodeWindow& w, NodePair& p,
+                                           const uint32_t* __restrict__ lcnt, uint32_t n,
+                                           const uint32_t* __restrict__ order, uint32_t lane) {
+  while (w.rest == 0) {
+    if (w.next >= n) return false;
+    const uint32_t c = w.next + lane * gridDim.x;
+    w.node = c < n ? (order ? __ldg(order + c) : c) : 0u;
+    w.cnt = make_uint2(0, 0);
+    if (c < n) w.cnt = *reinterpret_cast<const uint2*>(lcnt + 2 * (size_t)w.node);
+    w.rest = __ballot_sync(kFull, w.cnt.x > 0 && w.cnt.y >= 2);
+    w.small = __ballot_sync(kFull, w.cnt.y <= kMaxList / 2);
+    w.next += 32u * gridDim.x;
+  }
+  auto get = [&](int i, unsigned lanes) {
+    const int l = __ffs(lanes) - 1;
+    w.rest &= ~(1u << l);
+    p.u[i] = __shfl_sync(kFull, w.node, l);
+    p.nn[i] = __shfl_sync(kFull, w.cnt.x, l);
+    p.tot[i] = __shfl_sync(kFull, w.cnt.y, l);
+  };
+  get(0, w.rest);
+  p.u[1] = p.nn[1] = p.tot[1] = 0;
+  if (p.tot[0] <= kMaxList / 2 && (w.rest & w.small)) get(1, w.rest & w.small);
+  return true;
+}
+
+__device__ __forceinline__ void set_slot(NodeSlot& s, const NodePair& p) {
+  const bool two = p.tot[1] != 0;
+  s.live = 1;
+  s.first[0] = 0;
+  s.fresh[0] = p.nn[0];
+  s.total[0] = p.tot[0];
+  s.first[1] = two ? 2 : 0;
+  s.fresh[1] = two ? kMaxList / 2 + p.nn[1] : p.nn[0];
+  s.total[1] = two ? kMaxList / 2 + p.tot[1] : p.tot[0];
+}
+
+// Ids, norms and k-th distances of the tile's rows, by the producer warp; columns
+// without a row get an infinite norm, which the screen never keeps.
+__device__ __forceinline__ void load_rows(const NodePair& p, const float2* __restrict__ meta,
+                                          const uint32_t* __restrict__ lists, uint32_t lane,
+                                          uint32_t* ids, float* hnrm, float* kth) {
+  uint32_t id[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t t = lane + 32 * i, h = p.tot[1] && i >= 2;
+    const uint32_t at = t - h * (kMaxList / 2);
+    id[i] = at < (h ? p.tot[1] : p.tot[0])
+                ? __ldg(lists + (size_t)(h ? p.u[1] : p.u[0]) * kMaxList + at)
+                : kInv;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t t = lane + 32 * i;
+    float2 m = make_float2(INFINITY, 0.0f);
+    if (id[i] != kInv) {
+      m = __ldg(meta + id[i]);
+      m.x *= kOneMinusEps;
+    }
+    ids[t] = id[i];
+    hnrm[t] = m.x;
+    kth[t] = m.y;
+  }
+}
+
+// Bytes per 64-half column block of the tile's rows (groups of four), and lane's
+// four rows; false where its group has none.
+__device__ __forceinline__ uint32_t group_bytes(const NodePair& p) {
+  return ((p.tot[0] + 3) / 4 + (p.tot[1] + 3) / 4) * 4 * 128;
+}
+__device__ __forceinline__ bool group_rows(const NodePair& p, const uint32_t* ids, uint32_t lane,
+                                           uint32_t (&r)[4]) {
+  const bool h = p.tot[1] && lane >= 16;
+  const uint32_t end = h ? kMaxList / 2 + p.tot[1] : p.tot[0];
+  if (4 * lane >= end) return false;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) r[t] = ids[min(4 * lane + t, end - 1)];
+  return true;
+}
+
+// Producer warp: fills stage j % kStages with tile j (one node or two, take_nodes):
+// ids, norms and k-th distances (one packed record per row) by the lanes, rows by
+// TMA tile::gather4. Runs kStages tiles ahead of the consumers; ends by publishing
+// a slot that is not live.
 template <int D>
 __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* __restrict__ meta,
                               const uint32_t* __restrict__ lists,
@@ -288,10 +393,12 @@ __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* 
                               uint32_t K, unsigned long long* n_rows,
                               const uint32_t* __restrict__ order) {
   const uint32_t lane = threadIdx.x & 31u, blocks = (dim + 63) / 64;
-  uint32_t next = blockIdx.x;
+  NodeWindow win{blockIdx.x};
   uint32_t ph_empty[kStages] = {};
   for (uint32_t j = 0;; ++j) {
     const int st = (int)(j % kStages);
+    NodePair p;
+    const bool more = take_nodes(win, p, lcnt, n, order, lane);
     if (j >= (uint32_t)kStages) {
       bool ok = true;
       if (lane == 0) {
@@ -302,58 +409,29 @@ __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* 
       if (!__shfl_sync(kFull, ok ? 1 : 0, 0)) return;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    // next node with a join: 32 positions of the order per step, one per lane
-    uint32_t u = kDone, nn = 0, tot = 0;
-    while (next < n) {
-      const uint32_t c = next + lane * gridDim.x;
-      const uint32_t node = c < n ? (order ? __ldg(order + c) : c) : 0u;
-      uint2 cnt = make_uint2(0, 0);
-      if (c < n) cnt = *reinterpret_cast<const uint2*>(lcnt + 2 * (size_t)node);
-      const unsigned ok = __ballot_sync(kFull, c < n && cnt.x > 0 && cnt.y >= 2);
-      if (ok) {
-        const int w = __ffs(ok) - 1;
-        u = __shfl_sync(kFull, node, w);
-        nn = __shfl_sync(kFull, cnt.x, w);
-        tot = __shfl_sync(kFull, cnt.y, w);
-        next += ((uint32_t)w + 1u) * gridDim.x;
-        break;
+    const uint32_t bar = smem_u32(&s.full_bar[st]);
+    if (!more) {
+      if (lane == 0) {
+        s.slot[st].live = 0;
+        mbar_arrive(bar);
       }
-      next += 32u * gridDim.x;
-    }
-    if (lane == 0) {
-      s.node[st] = u;
-      s.nn[st] = nn;
-      s.total[st] = tot;
-    }
-    if (u == kDone) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s.full_bar[st]));
       return;
     }
-    for (uint32_t t = lane; t < tot; t += 32) {
-      const uint32_t id = lists[(size_t)u * kMaxList + t];
-      s.ids[st][t] = id;
-      const float2 m = __ldg(meta + id);
-      s.hnrm[st][t] = kOneMinusEps * m.x;
-      s.kth[st][t] = m.y;
-    }
-    for (uint32_t t = tot + lane; t < kMaxList; t += 32) s.hnrm[st][t] = INFINITY;
+    if (lane == 0) set_slot(s.slot[st], p);
+    load_rows(p, meta, lists, lane, s.ids[st], s.hnrm[st], s.kth[st]);
     __syncwarp();
-    const uint32_t groups = (tot + 3) / 4, bar = smem_u32(&s.full_bar[st]);
     if (lane == 0) {
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                   "r"(groups * 4 * 128 * blocks)
+                   "r"(group_bytes(p) * blocks)
                    : "memory");
-      *n_rows += tot;
+      *n_rows += p.tot[0] + p.tot[1];
       s.filled = j + 1;
     }
     __syncwarp();
-    for (uint32_t g = lane; g < groups; g += 32) {
-      uint32_t r[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) r[t] = s.ids[st][min(4 * g + t, tot - 1)];
+    uint32_t r[4];
+    if (group_rows(p, s.ids[st], lane, r)) {
       for (uint32_t b = 0; b < blocks; ++b) {
-        const uint32_t dst = smem_u32(&s.tile[st].x[b][4 * g][0]);
+        const uint32_t dst = smem_u32(&s.tile[st].x[b][4 * lane][0]);
         asm volatile(
             "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::"
             "bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
@@ -417,13 +495,13 @@ __global__ void __launch_bounds__(kThreads, 3)
     uint32_t ph_full[kStages] = {}, ph_mma[2] = {0, 0};
     bool pending[2] = {false, false};  // thread 0: committed MMAs not yet waited for
     // Thread 0: waits for stage st's rows (phase ph) and issues their Gram
-    // tile into accumulator acc. No MMA for a kDone stage or on timeout.
+    // tile into accumulator acc. No MMA for a stage that is not live or on timeout.
     auto issue = [&](int st, uint32_t ph, uint32_t acc) {
       if (!mbar_wait_bounded(smem_u32(&s.full_bar[st]), ph)) {
         s.flag = 0;
         return;
       }
-      if (s.node[st] == kDone) return;
+      if (!s.slot[st].live) return;
       asm volatile("tcgen05.fence::after_thread_sync;");
       for (uint32_t k = 0; k < ksteps; ++k) {
         const uint64_t desc = sw128_desc(smem_u32(&s.tile[st].x[k >> 2][0][0]) + (k & 3u) * 32);
@@ -447,24 +525,23 @@ __global__ void __launch_bounds__(kThreads, 3)
       const bool got = mbar_wait_bounded(smem_u32(&s.full_bar[st]), ph_full[st]);
       ph_full[st] ^= 1u;
       got_full += got ? 1u : 0u;
-      const bool done = got && s.node[st] == kDone;
+      const bool done = got && !s.slot[st].live;
       bool ok = got;
       if (got && !done) {
         ok = mbar_wait_bounded(smem_u32(&s.mma_bar[acc]), ph_mma[acc]);
         ph_mma[acc] ^= 1u;
         pending[acc] = false;
       }
-      // every consumer leaves together: on any thread's timeout, or at kDone
+      // every consumer leaves together: on any thread's timeout, or at the end
       if (consumers_any(!ok)) {
         if (tid == 0) s.flag = 0;
         break;
       }
       if (done) break;
-      const uint32_t nn = s.nn[st], total = s.total[st];
       asm volatile("tcgen05.fence::after_thread_sync;");
       // ---- screen: each thread owns one row ----
       uint32_t bc[4];
-      screen_rows(T, tmem + acc * 128, s.hnrm[st], s.hnrm[st][r], s.kth[st][r], r, nn, total, bc);
+      screen_rows(T, tmem + acc * 128, s.hnrm[st], s.hnrm[st][r], s.kth[st][r], r, s.slot[st], bc);
       // kept pairs go to one list so that the exact re-rank is shared evenly
       uint32_t kept = 0;
 #pragma unroll
@@ -561,13 +638,13 @@ struct __align__(1024) WideSmem {
   unsigned long long node_full[kWideNodes], node_empty[kWideNodes];
   unsigned long long acc_full[2], acc_empty[2], drain;
   uint32_t taddr;
-  uint32_t node[kWideNodes], nn[kWideNodes], total[kWideNodes];
+  NodeSlot slot[kWideNodes];
   uint32_t filled, taken;  // column blocks the producer issued / the MMA warp waited for
   int flag;
 };
 
-// Producer warp of the wide join: node metadata into slot j % 2, then the
-// node's column blocks, each into the next ring stage once the MMAs that read
+// Producer warp of the wide join: the metadata of tile j (one node or two,
+// take_nodes) into slot j % 2, then its column blocks, each into the next ring stage once the MMAs that read
 // it before have completed.
 __device__ void wide_producer(WideSmem& s, const CUtensorMap& tmap, const float2* __restrict__ meta,
                               const uint32_t* __restrict__ lists,
@@ -575,10 +652,13 @@ __device__ void wide_producer(WideSmem& s, const CUtensorMap& tmap, const float2
                               uint32_t K, unsigned long long* n_rows,
                               const uint32_t* __restrict__ order) {
   const uint32_t lane = threadIdx.x & 31u, blocks = (dim + 63) / 64;
-  uint32_t next = blockIdx.x, fill = 0;
+  NodeWindow win{blockIdx.x};
+  uint32_t fill = 0;
   uint32_t ph_node[kWideNodes] = {};
   for (uint32_t j = 0;; ++j) {
     const int ns = (int)(j % kWideNodes);
+    NodePair p;
+    const bool more = take_nodes(win, p, lcnt, n, order, lane);
     if (j >= (uint32_t)kWideNodes) {
       bool ok = true;
       if (lane == 0) {
@@ -588,41 +668,22 @@ __device__ void wide_producer(WideSmem& s, const CUtensorMap& tmap, const float2
       ph_node[ns] ^= 1u;
       if (!__shfl_sync(kFull, ok ? 1 : 0, 0)) return;
     }
-    uint32_t u = kDone, nn = 0, tot = 0;
-    while (next < n) {
-      const uint32_t c = next + lane * gridDim.x;
-      const uint32_t node = c < n ? (order ? __ldg(order + c) : c) : 0u;
-      uint2 cnt = make_uint2(0, 0);
-      if (c < n) cnt = *reinterpret_cast<const uint2*>(lcnt + 2 * (size_t)node);
-      const unsigned ok = __ballot_sync(kFull, c < n && cnt.x > 0 && cnt.y >= 2);
-      if (ok) {
-        const int w = __ffs(ok) - 1;
-        u = __shfl_sync(kFull, node, w);
-        nn = __shfl_sync(kFull, cnt.x, w);
-        tot = __shfl_sync(kFull, cnt.y, w);
-        next += ((uint32_t)w + 1u) * gridDim.x;
-        break;
+    if (!more) {
+      if (lane == 0) {
+        s.slot[ns].live = 0;
+        mbar_arrive(smem_u32(&s.node_full[ns]));
       }
-      next += 32u * gridDim.x;
+      return;
     }
-    for (uint32_t t = lane; t < tot; t += 32) {
-      const uint32_t id = lists[(size_t)u * kMaxList + t];
-      s.ids[ns][t] = id;
-      const float2 m = __ldg(meta + id);
-      s.hnrm[ns][t] = kOneMinusEps * m.x;
-      s.kth[ns][t] = m.y;
-    }
-    for (uint32_t t = tot + lane; t < kMaxList; t += 32) s.hnrm[ns][t] = INFINITY;
     if (lane == 0) {
-      s.node[ns] = u;
-      s.nn[ns] = nn;
-      s.total[ns] = tot;
+      set_slot(s.slot[ns], p);
+      *n_rows += p.tot[0] + p.tot[1];
     }
+    load_rows(p, meta, lists, lane, s.ids[ns], s.hnrm[ns], s.kth[ns]);
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&s.node_full[ns]));
-    if (u == kDone) return;
-    if (lane == 0) *n_rows += tot;
-    const uint32_t groups = (tot + 3) / 4;
+    uint32_t r[4];
+    const bool mine = group_rows(p, s.ids[ns], lane, r);
     for (uint32_t b = 0; b < blocks; ++b, ++fill) {
       const int slot = (int)(fill % kWideRing);
       const uint32_t bar = smem_u32(&s.ring_full[slot]);
@@ -634,17 +695,14 @@ __device__ void wide_producer(WideSmem& s, const CUtensorMap& tmap, const float2
           s.flag = 0;
         } else {
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                       "r"(groups * 4 * 128)
+                       "r"(group_bytes(p))
                        : "memory");
           s.filled = fill + 1;
         }
       }
       if (!__shfl_sync(kFull, ok ? 1 : 0, 0)) return;
-      for (uint32_t g = lane; g < groups; g += 32) {
-        uint32_t r[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) r[t] = s.ids[ns][min(4 * g + t, tot - 1)];
-        const uint32_t dst = smem_u32(&s.ring[slot][4 * g][0]);
+      if (mine) {
+        const uint32_t dst = smem_u32(&s.ring[slot][4 * lane][0]);
         asm volatile(
             "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::"
             "bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
@@ -668,8 +726,8 @@ __device__ void wide_mma(WideSmem& s, uint32_t tmem, uint32_t dim) {
       break;
     }
     ph_node[ns] ^= 1u;
-    if (s.node[ns] == kDone) {
-      mbar_arrive(smem_u32(&s.acc_full[acc]));  // wakes the consumers, who see kDone
+    if (!s.slot[ns].live) {
+      mbar_arrive(smem_u32(&s.acc_full[acc]));  // wakes the consumers, who see it too
       break;
     }
     if (j >= 2) {
@@ -768,17 +826,16 @@ __global__ void __launch_bounds__(kWideThreads, 2)
       ph_node[ns] ^= 1u;
       if (ok) ok = mbar_wait_bounded(smem_u32(&s.acc_full[acc]), ph_acc[acc]);
       ph_acc[acc] ^= 1u;
-      // every consumer leaves together: on any thread's timeout, or at kDone
+      // every consumer leaves together: on any thread's timeout, or at the end
       if (consumers_any(!ok)) {
         if (tid == 0) s.flag = 0;
         break;
       }
-      if (s.node[ns] == kDone) break;
-      const uint32_t nn = s.nn[ns], total = s.total[ns];
+      if (!s.slot[ns].live) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
       // ---- screen: the same rule and order as k_join_tc ----
       uint32_t bc[4];
-      screen_rows(T, tmem + acc * 128, s.hnrm[ns], s.hnrm[ns][r], s.kth[ns][r], r, nn, total, bc);
+      screen_rows(T, tmem + acc * 128, s.hnrm[ns], s.hnrm[ns][r], s.kth[ns][r], r, s.slot[ns], bc);
       // the accumulator is read: the MMA warp may refill it with node i + 2
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();

@@ -424,6 +424,175 @@ static __device__ __noinline__ float row_dist(const __half* __restrict__ a,
   return __fadd_rn(x, y);
 }
 
+// Distances of up to 32 rows ids[0, m) (shared memory, m >= 1) to one query by a
+// warp, in the reference's lane order; lane l returns the one of row rows32_of(l).
+//
+// Four lanes share a row: lane j holds the 16-byte units j, j + 4, j + 8 and j + 12 of
+// every 16, so levels 1 and 2 of the tree (slots 16 and 8 apart) are its own sums and
+// level 5 (neighbouring slots) too. Levels 3 and 4 exchange with lanes j ^ 2 and j ^ 1;
+// a lane keeps the half of its rows that its bit names and passes the other on, so
+// that 12 exchanges serve 32 rows and each lane ends with one.
+//
+// A lane per row, as before, touches 32 lines with each load: at 200K x 128 the L1 pipe
+// was 78 % busy and bounded the collect, and its unrolled tree left the instruction
+// cache. Eight lanes per row read whole lines, but their third exchange and half empty
+// loads at 96 dims took 1.8 times the instructions.
+// Collect with these, chained membership and rolled sorts: 1M x 128, K = 96, 98.4 ->
+// 79.6 ms; 500K x 96, K = 64, 32.1 -> 29.4 ms.
+__device__ __forceinline__ uint32_t rows32_of(int lane) {
+  return 8 * ((uint32_t)lane & 3u) + ((uint32_t)lane >> 2);
+}
+
+__device__ __forceinline__ void unit_acc(uint4 v, const float2 (&q)[4], float (&x)[2],
+                                         float (&y)[2]) {
+  float d0, d1, d2, d3;
+  sub_h2(v.x, q[0].x, q[0].y, d0, d1);
+  sub_h2(v.y, q[1].x, q[1].y, d2, d3);
+  fma2_sq(x[0], y[0], d0, d1);
+  fma2_sq(x[0], y[0], d2, d3);
+  sub_h2(v.z, q[2].x, q[2].y, d0, d1);
+  sub_h2(v.w, q[3].x, q[3].y, d2, d3);
+  fma2_sq(x[1], y[1], d0, d1);
+  fma2_sq(x[1], y[1], d2, d3);
+}
+__device__ __forceinline__ void widen(uint4 v, float2 (&q)[4]) {
+  q[0] = h2lo(v.x);
+  q[1] = h2lo(v.y);
+  q[2] = h2lo(v.z);
+  q[3] = h2lo(v.w);
+}
+// Keeps row a's sums (b's where `up`) and adds the partner's of the same row.
+__device__ __forceinline__ void pass_half(float (&xa)[2], float (&ya)[2], const float (&xb)[2],
+                                          const float (&yb)[2], bool up, int off) {
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const float kx = up ? xb[s] : xa[s], sx = up ? xa[s] : xb[s];
+    const float ky = up ? yb[s] : ya[s], sy = up ? ya[s] : yb[s];
+    xa[s] = kx;
+    ya[s] = ky;
+    add2(xa[s], ya[s], __shfl_xor_sync(kFull, sx, off), __shfl_xor_sync(kFull, sy, off));
+  }
+}
+
+// Rows of D = 96 or 128 halves (one chunk per slot).
+template <int D>
+__device__ __forceinline__ float warp_rows32_fixed(const __half* q, const __half* __restrict__ base,
+                                                   const uint32_t* ids, uint32_t m) {
+  static_assert(D == 96 || D == 128, "whole units of four lanes");
+  constexpr int U = D / 32;  // units per lane
+  const uint32_t lane = threadIdx.x & 31u, g = lane >> 2, j = lane & 3u;
+  const uint4* Q = reinterpret_cast<const uint4*>(q) + j;
+  const uint4* R[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    R[i] = reinterpret_cast<const uint4*>(base + (size_t)ids[min(8u * i + g, m - 1)] * D) + j;
+  float x[4][2], y[4][2];
+  // units k and k + 2 are level 1, the two sums level 2; slots without a chunk add
+  // an exact zero
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float2 q0[4], q1[4];
+    widen(__ldg(Q + 4 * h), q0);
+    if (h + 2 < U) widen(__ldg(Q + 4 * (h + 2)), q1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (8u * i >= m) break;
+      const uint4 v0 = __ldg(R[i] + 4 * h);
+      uint4 v1 = v0;
+      if (h + 2 < U) v1 = __ldg(R[i] + 4 * (h + 2));
+      float x0[2] = {0.0f, 0.0f}, y0[2] = {0.0f, 0.0f};
+      unit_acc(v0, q0, x0, y0);
+      if (h + 2 < U) {
+        float x1[2] = {0.0f, 0.0f}, y1[2] = {0.0f, 0.0f};
+        unit_acc(v1, q1, x1, y1);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) add2(x0[s], y0[s], x1[s], y1[s]);
+      }
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (h == 0) {
+          x[i][s] = x0[s];
+          y[i][s] = y0[s];
+        } else {
+          add2(x[i][s], y[i][s], x0[s], y0[s]);
+        }
+      }
+    }
+  }
+  pass_half(x[0], y[0], x[2], y[2], j & 2u, 2);
+  pass_half(x[1], y[1], x[3], y[3], j & 2u, 2);
+  pass_half(x[0], y[0], x[1], y[1], j & 1u, 1);
+  add2(x[0][0], y[0][0], x[0][1], y[0][1]);
+  return __fadd_rn(x[0][0], y[0][0]);
+}
+
+// Any width that is a multiple of four, 16 rows at a time.
+static __device__ __noinline__ float warp_rows32_any(const __half* q,
+                                                     const __half* __restrict__ base, uint32_t dim,
+                                                     const uint32_t* ids, uint32_t m) {
+  const uint32_t lane = threadIdx.x & 31u, g = lane >> 2, j = lane & 3u;
+  const uint32_t chunks = dim >> 2, units = (dim + 7) >> 3;
+  const bool aligned = (dim & 7u) == 0;
+  auto unit = [&](const __half* row, uint32_t u) {
+    if (aligned) return __ldg(reinterpret_cast<const uint4*>(row) + u);
+    const uint2* r = reinterpret_cast<const uint2*>(row);
+    const uint2 a = __ldg(r + 2 * u);
+    const uint2 b = 2 * u + 1 < chunks ? __ldg(r + 2 * u + 1) : make_uint2(0u, 0u);
+    return make_uint4(a.x, a.y, b.x, b.y);
+  };
+  float half[2] = {0.0f, 0.0f};
+#pragma unroll 1
+  for (uint32_t b = 0; b < 2 && 16 * b < m; ++b) {
+    const __half* R0 = base + (size_t)ids[min(16 * b + g, m - 1)] * dim;
+    const __half* R1 = base + (size_t)ids[min(16 * b + 8 + g, m - 1)] * dim;
+    float x[2][4][2], y[2][4][2];  // row, unit of the lane, slot of the unit
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) x[0][k][s] = y[0][k][s] = x[1][k][s] = y[1][k][s] = 0.0f;
+#pragma unroll 1
+    for (uint32_t u0 = 0; u0 < units; u0 += 16) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t u = u0 + 4 * k + j;
+        if (u < units) {
+          float2 qf[4];
+          widen(unit(q, u), qf);
+          unit_acc(unit(R0, u), qf, x[0][k], y[0][k]);
+          unit_acc(unit(R1, u), qf, x[1][k], y[1][k]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        add2(x[i][0][s], y[i][0][s], x[i][2][s], y[i][2][s]);
+        add2(x[i][1][s], y[i][1][s], x[i][3][s], y[i][3][s]);
+        add2(x[i][0][s], y[i][0][s], x[i][1][s], y[i][1][s]);
+      }
+    pass_half(x[0][0], y[0][0], x[1][0], y[1][0], j & 2u, 2);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const float ox = __shfl_xor_sync(kFull, x[0][0][s], 1),
+                  oy = __shfl_xor_sync(kFull, y[0][0][s], 1);
+      add2(x[0][0][s], y[0][0][s], ox, oy);
+    }
+    add2(x[0][0][0], y[0][0][0], x[0][0][1], y[0][0][1]);
+    half[b] = __fadd_rn(x[0][0][0], y[0][0][0]);  // row 16 b + 8 (j / 2) + g
+  }
+  const float lo = __shfl_sync(kFull, half[0], (int)((lane & ~3u) + 2 * (j & 1u)));
+  const float hi = __shfl_sync(kFull, half[1], (int)((lane & ~3u) + 2 * (j & 1u)));
+  return j < 2 ? lo : hi;
+}
+
+__device__ __forceinline__ float warp_rows32(const __half* q, const __half* __restrict__ base,
+                                             uint32_t dim, const uint32_t* ids, uint32_t m) {
+  if (dim == 128) return warp_rows32_fixed<128>(q, base, ids, m);
+  if (dim == 96) return warp_rows32_fixed<96>(q, base, ids, m);
+  return warp_rows32_any(q, base, dim, ids, m);
+}
+
 // distance_filter (src/Tagore_src.cu:1488-1490) as nvcc compiles it, one fused
 // multiply-add, and angle_filter (:1493-1495) with IEEE-rounded operations.
 __device__ __forceinline__ bool pruned_by(int metric, float res, float dis, float cur, float thre) {

@@ -37,77 +37,76 @@ constexpr int kWarps = 4;  // warps (= nodes in flight) per block
 // ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // Beam search shared by cal_ep_gpu (:1905-2047) and collect_path (:1211-1335).
-// The helpers below are __noinline__: the select kernel is latency-bound and
-// its warps sit in different phases, so one copy of each sort and merge keeps
-// the code they run small enough for the instruction cache (inlined copies
-// at every call site cost 8 % of the select at 1M points).
+// The helpers below are __noinline__ and their sorts rolled: the warps sit in
+// different phases, so one small copy of each sort and merge keeps the code they
+// run within the instruction cache. Inlined copies at every call site cost 8 % of
+// the select at 1M points; the sorts with their passes unrolled, 10.6 of the
+// collect's 89.8 ms.
 struct Beam {
   uint32_t* id;
   float* dis;
   uint8_t* ex;
-  uint32_t* hash;  // membership set of the W beam ids (open addressing)
-  uint32_t hslots;  // hash slots
+  // membership set of the W beam ids, as chains: heads, the ids as they were when
+  // the set was made, and links
+  uint32_t *head, *nid;
+  uint16_t* next;
   float* sb;       // scratch (K): the fresh positions, then sorted entering distances
-  float* sm;       // staging (W + 1): merged distances of positions 0..TOPM
-  uint32_t* sid;   // staging (W + 1): their ids
-  uint8_t* sex;    // staging (W + 1): their explored flags
+  float* sm;       // staging: merged distances of positions 0..TOPM, or K entering ones
+  uint32_t* sid;   // staging: their ids
+  uint8_t* sex;    // staging: their explored flags
 };
 
-// Hash slots: the beam at load <= 1/2 (TOPM <= 256, K <= 128). 384 slots keep a
-// warp's beam region within its candidate list's, so six blocks per SM still
-// fit the 132 KB shared-memory carveout and leave L1 its larger share.
-__host__ __device__ inline uint32_t hash_slots(uint32_t W) { return W <= 192 ? 384u : 768u; }
+constexpr uint32_t kBeamHeads = 256;
 
-__host__ __device__ inline size_t beam_bytes(uint32_t W) {
-  return (size_t)hash_slots(W) * 4 + (size_t)W * 8 + 128 * 4 + (size_t)(W + 1) * 8 +
-         ((W + 15u) & ~15u) + ((W + 16u) & ~15u);
+__host__ __device__ inline size_t beam_bytes(uint32_t topm, uint32_t K) {
+  const uint32_t W = topm + K, S = topm + 1 > K ? topm + 1 : K;
+  return kBeamHeads * 4 + (size_t)W * 12 + K * 4 + (size_t)S * 8 + ((W * 2 + 3u) & ~3u) + W +
+         topm + 1;
 }
 
-__device__ inline Beam beam_carve(unsigned char* p, uint32_t W) {
+__device__ inline Beam beam_carve(unsigned char* p, uint32_t topm, uint32_t K) {
+  const uint32_t W = topm + K, S = topm + 1 > K ? topm + 1 : K;
   Beam b;
-  b.hash = reinterpret_cast<uint32_t*>(p);
-  b.hslots = hash_slots(W);
-  b.id = b.hash + hash_slots(W);
+  b.head = reinterpret_cast<uint32_t*>(p);
+  b.id = b.head + kBeamHeads;
   b.dis = reinterpret_cast<float*>(b.id + W);
-  b.sb = b.dis + W;
-  b.sm = b.sb + 128;
-  b.sid = reinterpret_cast<uint32_t*>(b.sm + W + 1);
-  b.ex = reinterpret_cast<uint8_t*>(b.sid + W + 1);
-  b.sex = b.ex + ((W + 15u) & ~15u);
+  b.nid = reinterpret_cast<uint32_t*>(b.dis + W);
+  b.sb = reinterpret_cast<float*>(b.nid + W);
+  b.sm = b.sb + K;
+  b.sid = reinterpret_cast<uint32_t*>(b.sm + S);
+  b.next = reinterpret_cast<uint16_t*>(b.sid + S);
+  b.ex = reinterpret_cast<uint8_t*>(b.next) + ((W * 2 + 3u) & ~3u);
+  b.sex = b.ex + W;
   return b;
 }
 
-__device__ __forceinline__ uint32_t hslot(uint32_t key, uint32_t slots) {
-  return (uint32_t)(((uint64_t)(key * 0x9E3779B1u) * slots) >> 32);  // multiply-shift into [0, slots)
-}
+__device__ __forceinline__ uint32_t beam_head(uint32_t key) { return (key * 0x9E3779B1u) >> 24; }
 
 // The reference keeps the beam ids sorted (top_M_Cand2, :1253-1259) only to
-// test membership (:1282-1290); a hash set of the same ids answers the same
-// question without a sort.
+// test membership (:1282-1290); a set of the same ids answers the same question
+// without a sort. Chains take one exchange per id, where a probed table's 32
+// lanes wait for the longest run of tries among them.
 __device__ __noinline__ void beam_rehash(Beam bm, uint32_t W, int lane) {
-  for (uint32_t t = lane; t < bm.hslots; t += 32) bm.hash[t] = kInv;
+#pragma unroll
+  for (uint32_t t = lane; t < kBeamHeads / 4; t += 32)
+    reinterpret_cast<uint4*>(bm.head)[t] = make_uint4(kInv, kInv, kInv, kInv);
   __syncwarp();
   for (uint32_t t = lane; t < W; t += 32) {
     const uint32_t key = bm.id[t];
     if (key == kInv) continue;
-    uint32_t h = hslot(key, bm.hslots);
-    while (true) {
-      const uint32_t prev = atomicCAS(&bm.hash[h], kInv, key);
-      if (prev == kInv || prev == key) break;
-      h = h + 1 == bm.hslots ? 0u : h + 1;
-    }
+    bm.nid[t] = key;
+    bm.next[t] = (uint16_t)atomicExch(&bm.head[beam_head(key)], t);
   }
   __syncwarp();
 }
 
 __device__ __forceinline__ bool beam_has(const Beam& bm, uint32_t key) {
-  uint32_t h = hslot(key, bm.hslots);
-  while (true) {
-    const uint32_t v = bm.hash[h];
-    if (v == key) return true;
-    if (v == kInv) return false;
-    h = h + 1 == bm.hslots ? 0u : h + 1;
+  uint32_t t = bm.head[beam_head(key)];
+  while ((t & 0xFFFFu) != 0xFFFFu) {
+    if (bm.nid[t] == key) return true;
+    t = bm.next[t];
   }
+  return false;
 }
 
 __device__ __noinline__ void beam_network(Beam bm, uint32_t off, uint32_t len, int lane) {
@@ -131,7 +130,7 @@ __device__ __forceinline__ void sorted_keys(const Beam& bm, uint32_t off, uint32
     const uint32_t j = lane + 32 * t;
     key[t] = j < n ? (((uint64_t)__float_as_uint(bm.dis[off + j]) << 32) | j) : ~0ull;
   }
-  knn::warp_sort_keys<4>(key, lane);
+  knn::warp_sort_keys_rolled<4>(key, lane);
 }
 
 __device__ __forceinline__ float key_dis(uint64_t k) { return __uint_as_float((uint32_t)(k >> 32)); }
@@ -147,7 +146,7 @@ __device__ __noinline__ bool beam_merge(Beam bm, uint32_t topm, uint32_t m, int 
     const uint32_t q = lane + 32 * t;
     key[t] = q < m ? (((uint64_t)__float_as_uint(bm.sm[q]) << 32) | bm.sid[q]) : ~0ull;
   }
-  knn::warp_sort_keys<E>(key, lane);
+  knn::warp_sort_keys_rolled<E>(key, lane);
 #pragma unroll
   for (int t = 0; t < E; ++t) {
     const uint32_t q = lane + 32 * t;
@@ -261,123 +260,125 @@ __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __re
     bm.ex[t] = 1;
   }
   __syncwarp();
-  // Seeds: the start node's row, scored one row per lane; ring slots follow
-  // the row order.
-  for (uint32_t t = lane; t < K; t += 32) {
-    const uint32_t a = __ldg(G + (size_t)start * K + t);
-    const float d = row_dist(query, data + (size_t)a * dim, dim);
-    bm.id[topm + t] = a;
-    bm.ex[topm + t] = 0;
-    bm.dis[topm + t] = d;
-    if (ring_id) {
-      ring_id[t % kSelectCand] = a;
-      ring_dis[t % kSelectCand] = d;
-    }
-  }
-  __syncwarp();
-  // Seeds: the network's order is observable on the first min(TOPM, K)
-  // positions, copied into the prefix; a tie there runs the network.
-  const uint32_t keep = min(topm, K);
-  bool seeded = false;
-  if (K <= 128) {
-    uint64_t key[4];
-    sorted_keys(bm, topm, K, key, lane);
-    bool tie = false;
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const uint32_t p = lane + 32 * t;
-      uint32_t prev = __shfl_up_sync(kFull, (uint32_t)(key[t] >> 32), 1);
-      if (t > 0) {
-        const uint32_t tail = __shfl_sync(kFull, (uint32_t)(key[t - 1] >> 32), 31);
-        if (lane == 0) prev = tail;
-      }
-      if (p >= 1 && p <= keep && p < K && (uint32_t)(key[t] >> 32) == prev) tie = true;
-    }
-    if (!__any_sync(kFull, tie)) {
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint32_t p = lane + 32 * t;
-        if (p < keep) {
-          const uint32_t j = (uint32_t)(key[t] & 0xFFFFFFFFu);
-          bm.id[p] = bm.id[topm + j];
-          bm.dis[p] = key_dis(key[t]);
-          bm.ex[p] = 0;
+  const uint32_t own = rows32_of(lane);
+  uint32_t* fresh_at = reinterpret_cast<uint32_t*>(bm.sb);  // K <= 128 slots
+  uint32_t curr = 0, to_explore = start;
+  // Round 0 scores the start node's whole row (the seeds), the later ones the
+  // neighbours of an explored node that are not in the beam.
+  for (uint32_t it = 0; it <= iters; ++it) {
+    if (it > 0) {
+      // First unexplored of the top TOPM; when none is left the reference keeps
+      // the previous node (its `j == TOPM` test never fires, :1270).
+      for (uint32_t base = 0; base < topm; base += 32) {
+        const uint32_t j = base + lane;
+        const unsigned m = __ballot_sync(kFull, j < topm && !bm.ex[j]);
+        if (m) {
+          const uint32_t f = base + __ffs(m) - 1;
+          to_explore = bm.id[f];
+          __syncwarp();
+          if (lane == 0) bm.ex[f] = 1;
+          break;
         }
       }
-      for (uint32_t i = K + lane; i < topm; i += 32) {  // TOPM > K: empty slots
-        bm.id[i] = kInv;
-        bm.dis[i] = kInfDis;
-        bm.ex[i] = 1;
-      }
-      seeded = true;
+      __syncwarp();
+      if (to_explore == kInv) break;
     }
-  }
-  if (!seeded) {
-    beam_network(bm, topm, K, lane);
-    for (uint32_t i = lane; i < topm; i += 32) {
-      if (topm + i < W) {
-        bm.id[i] = bm.id[topm + i];
-        bm.dis[i] = bm.dis[topm + i];
-        bm.ex[i] = bm.ex[topm + i];
-      } else {  // slots past the K seeds start empty (TOPM > K)
-        bm.id[i] = kInv;
-        bm.dis[i] = kInfDis;
-        bm.ex[i] = 1;
-      }
-    }
-  }
-  __syncwarp();
-  beam_rehash(bm, W, lane);
-  uint32_t curr = K, to_explore = kInv;
-  for (uint32_t it = 0; it < iters; ++it) {
-    // First unexplored of the top TOPM; when none is left the reference keeps
-    // the previous node (its `j == TOPM` test never fires, :1270).
-    for (uint32_t base = 0; base < topm; base += 32) {
-      const uint32_t j = base + lane;
-      const unsigned m = __ballot_sync(kFull, j < topm && !bm.ex[j]);
-      if (m) {
-        const uint32_t f = base + __ffs(m) - 1;
-        to_explore = bm.id[f];
-        __syncwarp();
-        if (lane == 0) bm.ex[f] = 1;
-        break;
-      }
-    }
-    __syncwarp();
-    if (to_explore == kInv) break;
-    // Neighbours of the explored node: members of the beam keep INF_DIS; the
-    // others are listed in ascending neighbour order (which fixes their ring
-    // slots) and scored one row per lane.
-    uint32_t* fresh_at = reinterpret_cast<uint32_t*>(bm.sb);  // K <= 128 slots
+    // Members of the beam keep INF_DIS; the others are listed in ascending
+    // neighbour order (which fixes their ring slots) and scored 32 at a time.
     uint32_t nfresh = 0;
     for (uint32_t base = 0; base < K; base += 32) {
       const uint32_t j = base + lane;
       bool fresh = false;
+      uint32_t a = kInv;
       if (j < K) {
-        const uint32_t a = __ldg(G + (size_t)to_explore * K + j);
-        fresh = !beam_has(bm, a);
+        a = __ldg(G + (size_t)to_explore * K + j);
+        fresh = it == 0 || !beam_has(bm, a);
         bm.id[topm + j] = a;
         bm.ex[topm + j] = 0;
         bm.dis[topm + j] = kInfDis;
       }
       const unsigned m = __ballot_sync(kFull, fresh);
-      if (fresh) fresh_at[nfresh + __popc(m & ((1u << lane) - 1u))] = j;
+      if (fresh) {
+        const uint32_t r = nfresh + __popc(m & ((1u << lane) - 1u));
+        fresh_at[r] = j;
+        bm.sid[r] = a;
+      }
       nfresh += __popc(m);
     }
     __syncwarp();
-    for (uint32_t r = lane; r < nfresh; r += 32) {
-      const uint32_t j = fresh_at[r];
-      const uint32_t a = bm.id[topm + j];
-      const float d = row_dist(query, data + (size_t)a * dim, dim);
-      bm.dis[topm + j] = d;
-      if (ring_id) {
-        ring_id[(curr + r) % kSelectCand] = a;
-        ring_dis[(curr + r) % kSelectCand] = d;
+    for (uint32_t base = 0; base < nfresh; base += 32) {
+      const uint32_t r = base + own;
+      const float d = warp_rows32(query, data, dim, bm.sid + base, min(32u, nfresh - base));
+      if (r < nfresh) {
+        bm.dis[topm + fresh_at[r]] = d;
+        if (ring_id) {
+          uint32_t p = curr + r;
+          while (p >= kSelectCand) p -= kSelectCand;
+          ring_id[p] = bm.sid[r];
+          ring_dis[p] = d;
+        }
       }
     }
     curr += nfresh;
     __syncwarp();
-    beam_update(bm, topm, K, fresh_at, nfresh, lane);
+    if (it > 0) {
+      beam_update(bm, topm, K, fresh_at, nfresh, lane);
+      continue;
+    }
+    // Seeds: the network's order is observable on the first min(TOPM, K)
+    // positions, copied into the prefix; a tie there runs the network.
+    const uint32_t keep = min(topm, K);
+    bool seeded = false;
+    if (K <= 128) {
+      uint64_t key[4];
+      sorted_keys(bm, topm, K, key, lane);
+      bool tie = false;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const uint32_t p = lane + 32 * t;
+        uint32_t prev = __shfl_up_sync(kFull, (uint32_t)(key[t] >> 32), 1);
+        if (t > 0) {
+          const uint32_t tail = __shfl_sync(kFull, (uint32_t)(key[t - 1] >> 32), 31);
+          if (lane == 0) prev = tail;
+        }
+        if (p >= 1 && p <= keep && p < K && (uint32_t)(key[t] >> 32) == prev) tie = true;
+      }
+      if (!__any_sync(kFull, tie)) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const uint32_t p = lane + 32 * t;
+          if (p < keep) {
+            const uint32_t j = (uint32_t)(key[t] & 0xFFFFFFFFu);
+            bm.id[p] = bm.id[topm + j];
+            bm.dis[p] = key_dis(key[t]);
+            bm.ex[p] = 0;
+          }
+        }
+        for (uint32_t i = K + lane; i < topm; i += 32) {  // TOPM > K: empty slots
+          bm.id[i] = kInv;
+          bm.dis[i] = kInfDis;
+          bm.ex[i] = 1;
+        }
+        seeded = true;
+      }
+    }
+    if (!seeded) {
+      beam_network(bm, topm, K, lane);
+      for (uint32_t i = lane; i < topm; i += 32) {
+        if (topm + i < W) {
+          bm.id[i] = bm.id[topm + i];
+          bm.dis[i] = bm.dis[topm + i];
+          bm.ex[i] = bm.ex[topm + i];
+        } else {  // slots past the K seeds start empty (TOPM > K)
+          bm.id[i] = kInv;
+          bm.dis[i] = kInfDis;
+          bm.ex[i] = 1;
+        }
+      }
+    }
+    __syncwarp();
+    beam_rehash(bm, W, lane);
+    to_explore = kInv;
   }
   if (ring_count) *ring_count = curr;
   return bm.id[0];
@@ -428,6 +429,169 @@ __device__ __forceinline__ uint32_t warp_compact(uint32_t* cand, float* dis, uin
   __syncwarp();
   *tail = len > 0 && ((ok >> ((len - 1) & 31u)) & 1u);
   return m;
+}
+
+// Words that mark the places of the kNN row's entries in the merged list.
+constexpr uint32_t kMarkWords = (kSelectCand + 128 + 31) / 32;
+
+// warp_sort_mark and warp_compact of a candidate list (K kNN entries, then
+// kSelectCand collected ones, in shared memory) where the order of equal
+// distances cannot be observed, written to out_ids / out_dis: the collected
+// entries are sorted in registers and merged with the row, which is sorted
+// already. Returns the entries left, or -1 where the network has to decide: a
+// row out of order, a distance that is negative or NaN, or equal distances of
+// different ids (entries with the same id and distance are the same in any
+// order). The collected part of the list is overwritten.
+//
+// Bound by instruction issue: about 3.5K instructions per warp against 7.6K of
+// the network, its marks and the compaction. The keys lie 16 to a lane, so that 30
+// of the 45 passes exchange within a lane; every merge starts mirrored, which
+// leaves one direction of comparison.
+// Collect at 500K x 96, K = 64: 29.1 ms with the network, 28.0 ms with this.
+__device__ __noinline__ int warp_list(uint32_t* cand, float* cdis, uint32_t* mark, uint32_t K,
+                                      uint32_t bid, uint32_t* __restrict__ out_ids,
+                                      float* __restrict__ out_dis, bool* tail, int lane) {
+  constexpr uint32_t kLast = 0x7F800000u;  // bits of +inf
+  constexpr int E = 16;
+  static_assert(kSelectCand == 30 * E, "the pads fill the last two lanes");
+  uint32_t key[E], id[E];
+  bool bad = false;
+#pragma unroll
+  for (int t = 0; t < E - 1; ++t) {
+    const uint32_t e = K + 32 * t + lane;
+    key[t] = __float_as_uint(cdis[e]);
+    id[t] = cand[e];
+    bad |= key[t] > kLast;
+  }
+  key[E - 1] = kInv;
+  id[E - 1] = kInv;
+  for (uint32_t i = lane; i < K; i += 32) {
+    const uint32_t k = __float_as_uint(cdis[i]);
+    bad |= k > kLast;
+    if (i > 0) {
+      const uint32_t p = __float_as_uint(cdis[i - 1]);
+      bad |= k < p || (k == p && cand[i] != cand[i - 1]);
+    }
+  }
+  if (__any_sync(kFull, bad)) return -1;
+  // ascending, position 16 * lane + t
+  auto in_lane = [&](int a, int b) {
+    const bool s = key[a] > key[b];
+    const uint32_t ka = key[a], kb = key[b], ia = id[a], ib = id[b];
+    key[a] = s ? kb : ka;
+    key[b] = s ? ka : kb;
+    id[a] = s ? ib : ia;
+    id[b] = s ? ia : ib;
+  };
+  auto take = [&](int a, uint32_t ok, uint32_t oi, bool upper) {
+    const bool s = upper ? ok > key[a] : ok < key[a];
+    key[a] = s ? ok : key[a];
+    id[a] = s ? oi : id[a];
+  };
+#pragma unroll
+  for (int size = 2; size <= E; size <<= 1) {
+#pragma unroll
+    for (int t = 0; t < E; ++t)
+      if (t < (t ^ (size - 1))) in_lane(t, t ^ (size - 1));
+#pragma unroll
+    for (int st = size / 4; st > 0; st >>= 1)
+#pragma unroll
+      for (int t = 0; t < E; ++t)
+        if (!(t & st)) in_lane(t, t | st);
+  }
+#pragma unroll 1
+  for (int lanes = 2; lanes <= 32; lanes <<= 1) {
+    const bool up = lane & (lanes >> 1);
+#pragma unroll
+    for (int t = 0; t < E / 2; ++t) {
+      const int q = E - 1 - t;
+      const uint32_t k0 = __shfl_xor_sync(kFull, key[q], lanes - 1);
+      const uint32_t i0 = __shfl_xor_sync(kFull, id[q], lanes - 1);
+      const uint32_t k1 = __shfl_xor_sync(kFull, key[t], lanes - 1);
+      const uint32_t i1 = __shfl_xor_sync(kFull, id[t], lanes - 1);
+      take(t, k0, i0, up);
+      take(q, k1, i1, up);
+    }
+#pragma unroll 1
+    for (int st = lanes >> 2; st > 0; st >>= 1) {
+      const bool upper = lane & st;
+#pragma unroll
+      for (int t = 0; t < E; ++t) {
+        const uint32_t ok = __shfl_xor_sync(kFull, key[t], st);
+        const uint32_t oi = __shfl_xor_sync(kFull, id[t], st);
+        take(t, ok, oi, upper);
+      }
+    }
+#pragma unroll
+    for (int st = E / 2; st > 0; st >>= 1)
+#pragma unroll
+      for (int t = 0; t < E; ++t)
+        if (!(t & st)) in_lane(t, t | st);
+  }
+#pragma unroll
+  for (int t = 0; t + 1 < E; ++t) bad |= key[t] == key[t + 1] && id[t] != id[t + 1];
+  {
+    const uint32_t nk = __shfl_down_sync(kFull, key[0], 1), ni = __shfl_down_sync(kFull, id[0], 1);
+    bad |= lane < 31 && key[E - 1] == nk && id[E - 1] != ni;
+  }
+  if (__any_sync(kFull, bad)) return -1;
+  // back to the list, the 16 places of a lane permuted against bank conflicts
+  auto place = [](uint32_t p) { return (p & ~15u) | ((p ^ (p >> 4)) & 15u); };
+  if (lane < 30) {
+#pragma unroll
+    for (int t = 0; t < E; ++t) {
+      const uint32_t e = K + place(lane * E + t);
+      cdis[e] = __uint_as_float(key[t]);
+      cand[e] = id[t];
+    }
+  }
+  if (lane < (int)kMarkWords) mark[lane] = 0;
+  __syncwarp();
+  for (uint32_t i = lane; i < K; i += 32) {
+    const uint32_t k = __float_as_uint(cdis[i]);
+    uint32_t lo = 0, hi = kSelectCand;  // collected entries before row entry i
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (__float_as_uint(cdis[K + place(mid)]) < k) lo = mid + 1;
+      else hi = mid;
+    }
+    if (lo < kSelectCand) {
+      const uint32_t e = K + place(lo);
+      bad |= __float_as_uint(cdis[e]) == k && cand[e] != cand[i];
+    }
+    const uint32_t f = i + lo;
+    atomicOr(&mark[f >> 5], 1u << (f & 31u));
+  }
+  if (__any_sync(kFull, bad)) return -1;
+  __syncwarp();
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t total = K + kSelectCand;
+  uint32_t rows = 0, m = 0, carry = kInv;
+  unsigned ok = 0;
+  for (uint32_t base = 0; base < total; base += 32) {
+    const uint32_t f = base + lane, w = mark[base >> 5], r = rows + __popc(w & below);
+    const uint32_t e = (w >> lane) & 1u ? r : K + place(f - r);
+    uint32_t c = kInv;
+    float d = 0.0f;
+    if (f < total) {
+      c = cand[e];
+      d = cdis[e];
+    }
+    uint32_t prev = __shfl_up_sync(kFull, c, 1);
+    if (lane == 0) prev = carry;
+    carry = __shfl_sync(kFull, c, 31);
+    const bool keep = c != kInv && c != bid && !(f >= 1 && c == prev);
+    ok = __ballot_sync(kFull, keep);
+    if (keep) {
+      const uint32_t p = m + __popc(ok & below);
+      out_ids[p] = c;
+      out_dis[p] = d;
+    }
+    m += __popc(ok);
+    rows += __popc(w);
+  }
+  *tail = (ok >> ((total - 1) & 31u)) & 1u;
+  return (int)m;
 }
 
 // Kept neighbours of one node, and the rows of a tile that outlived the kept
@@ -572,12 +736,13 @@ __device__ __forceinline__ uint32_t warp_filter(const uint32_t* cand, const floa
 // the candidate list share one region, since the list is filled only after
 // the beam has finished (its ring of scored nodes lives in global memory).
 struct SelLayout {
-  uint32_t W, L;
+  uint32_t topm, K;  // topm 0: no beam
   size_t tail;  // bytes behind the list (kept_bytes where the kernel also filters)
+  __host__ __device__ uint32_t L() const { return kSelectCand + K; }
   __host__ __device__ size_t bytes() const {
-    const size_t list = (size_t)L * 8 + tail;
-    const size_t beam = W ? beam_bytes(W) : 0;
-    return ((beam > list ? beam : list) + 64 + 15) & ~(size_t)15;
+    const size_t list = (size_t)L() * 8 + kMarkWords * 4 + tail;
+    const size_t beam = topm ? beam_bytes(topm, K) : 0;
+    return ((beam > list ? beam : list) + 15) & ~(size_t)15;
   }
 };
 
@@ -621,8 +786,7 @@ __global__ void k_cal_ep(const uint32_t* __restrict__ G, const __half* __restric
                          const __half* __restrict__ center, uint32_t dim, uint32_t K,
                          uint32_t topm, uint32_t* ep) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const uint32_t W = topm + K;
-  Beam bm = beam_carve(smem, W);
+  Beam bm = beam_carve(smem, topm, K);
   const int lane = threadIdx.x & 31;
   if (threadIdx.x >= 32) return;
   const uint32_t best = warp_beam(G, data, dim, K, center, 0, topm, 30, bm, nullptr, nullptr,
@@ -643,20 +807,20 @@ __device__ __forceinline__ uint32_t node_at(const uint32_t* __restrict__ order, 
 }
 
 // The collect half of select_path (:1498-1517) and select_2hop (:1520-1534):
-// node b's sorted candidate list (its kNN row and the collected nodes) without
-// repeats and b itself, in cand / cdis. Returns its length; *scored adds the
-// rows scored. rid / rds: this warp's ring of kSelectCand scored nodes (path).
+// node b's candidates (its kNN row and the collected nodes), unsorted, in
+// cand / cdis. Returns the rows scored. rid / rds: this warp's ring of kSelectCand
+// scored nodes (path).
 template <bool kPath>
 __device__ __forceinline__ uint32_t collect_node(
     const uint32_t* __restrict__ G, const float* __restrict__ nd, const __half* __restrict__ data,
     uint32_t dim, uint32_t K, uint32_t ep, uint32_t topm, uint32_t b, Beam bm, uint32_t* rid,
-    float* rds, uint32_t* cand, float* cdis, bool* tail, uint32_t* scored, int lane) {
+    float* rds, uint32_t* cand, float* cdis, int lane) {
   const __half* q = data + (size_t)b * dim;
-  *scored = kSelectCand;  // 2-hop: the 480 collected
+  uint32_t scored = kSelectCand;  // 2-hop: the 480 collected
   if (kPath) {
     uint32_t curr = 0;
     warp_beam(G, data, dim, K, q, ep, topm, 10, bm, rid, rds, &curr, lane);
-    *scored = curr;
+    scored = curr;
     __syncwarp();  // the ring (global) and the beam's region are done
     for (uint32_t i = lane; i < kSelectCand; i += 32) {
       const bool in = i < curr;
@@ -691,8 +855,7 @@ __device__ __forceinline__ uint32_t collect_node(
     cdis[i] = nd[(size_t)b * K + i];
   }
   __syncwarp();
-  warp_sort_mark(cand, cdis, kSelectCand + K, lane);
-  return warp_compact(cand, cdis, kSelectCand + K, b, tail, lane);
+  return scored;
 }
 
 // The filter half: select_path and select_2hop always use distance_filter and
@@ -729,7 +892,7 @@ __device__ __forceinline__ void filter_node(const uint32_t* cand, const float* c
 constexpr uint32_t kTailBit = 0x80000000u;
 
 template <bool kPath>
-__global__ void __launch_bounds__(kWarps * 32, 6)
+__global__ void __launch_bounds__(kWarps * 32, 7)
     k_collect(const uint32_t* __restrict__ G, const float* __restrict__ nd,
               const __half* __restrict__ data, uint32_t first, uint32_t cnt, uint32_t dim,
               uint32_t K, const uint32_t* __restrict__ ep_dev, uint32_t* __restrict__ ctr,
@@ -739,11 +902,12 @@ __global__ void __launch_bounds__(kWarps * 32, 6)
               const uint32_t* __restrict__ order) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const SelLayout lay{kPath ? topm + K : 0u, kSelectCand + K, 0};
+  const SelLayout lay{kPath ? topm : 0u, K, 0};
   unsigned char* mine = smem + (size_t)warp * lay.bytes();
   uint32_t* cand = reinterpret_cast<uint32_t*>(mine);
-  float* cdis = reinterpret_cast<float*>(cand + lay.L);
-  Beam bm = beam_carve(mine, lay.W);  // same region as the list, used before it
+  float* cdis = reinterpret_cast<float*>(cand + lay.L());
+  uint32_t* mark = reinterpret_cast<uint32_t*>(cdis + lay.L());
+  Beam bm = beam_carve(mine, lay.topm, K);  // same region as the list, used before it
   const size_t gw = (size_t)blockIdx.x * kWarps + warp;
   uint32_t* rid = kPath ? ring_ids + gw * kSelectCand : nullptr;
   float* rds = kPath ? ring_dis + gw * kSelectCand : nullptr;
@@ -752,14 +916,37 @@ __global__ void __launch_bounds__(kWarps * 32, 6)
   for (uint32_t i = next_node(ctr, lane); i < cnt; i = next_node(ctr, lane)) {
     const uint32_t b = node_at(order, first + i);
     bool tail = false;
-    uint32_t scored = 0;
-    const uint32_t len = collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand,
-                                             cdis, &tail, &scored, lane);
-    rows += scored + len;
-    for (uint32_t j = lane; j < len; j += 32) {
-      L_ids[(size_t)i * lay.L + j] = cand[j];
-      L_dis[(size_t)i * lay.L + j] = cdis[j];
+    const uint32_t scored =
+        collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
+    uint32_t* out_ids = L_ids + (size_t)i * lay.L();
+    float* out_dis = L_dis + (size_t)i * lay.L();
+    if (!kPath) {
+      // the collected entries' distances, should the network need them back
+      for (uint32_t j = lane; j < kSelectCand; j += 32) out_dis[j] = cdis[K + j];
+      __syncwarp();
     }
+    int got = warp_list(cand, cdis, mark, K, b, out_ids, out_dis, &tail, lane);
+    if (got < 0) {
+      // the list as it was collected, sorted by the network
+      for (uint32_t j = lane; j < kSelectCand; j += 32) {
+        if (kPath) {
+          cand[K + j] = j < scored ? rid[j] : kInv;
+          cdis[K + j] = j < scored ? rds[j] : kInfDis;
+        } else {
+          cand[K + j] = __ldg(G + (size_t)cand[j / K] * K + j % K);
+          cdis[K + j] = out_dis[j];
+        }
+      }
+      __syncwarp();
+      warp_sort_mark(cand, cdis, lay.L(), lane);
+      got = (int)warp_compact(cand, cdis, lay.L(), b, &tail, lane);
+      for (uint32_t j = lane; j < (uint32_t)got; j += 32) {
+        out_ids[j] = cand[j];
+        out_dis[j] = cdis[j];
+      }
+    }
+    const uint32_t len = (uint32_t)got;
+    rows += scored + len;
     if (lane == 0) L_cnt[i] = len | (tail ? kTailBit : 0u);
     __syncwarp();
   }
@@ -795,21 +982,21 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
              float* __restrict__ ring_dis) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const SelLayout lay{kPath ? topm + K : 0u, kSelectCand + K, kept_bytes(fd)};
+  const SelLayout lay{kPath ? topm : 0u, K, kept_bytes(fd)};
   unsigned char* mine = smem + (size_t)warp * lay.bytes();
   uint32_t* cand = reinterpret_cast<uint32_t*>(mine);
-  float* cdis = reinterpret_cast<float*>(cand + lay.L);
-  const Kept k = kept_carve(reinterpret_cast<unsigned char*>(cdis + lay.L), fd);
-  Beam bm = beam_carve(mine, lay.W);  // same region as the list, used before it
+  float* cdis = reinterpret_cast<float*>(cand + lay.L());
+  const Kept k = kept_carve(reinterpret_cast<unsigned char*>(cdis + lay.L()) + kMarkWords * 4, fd);
+  Beam bm = beam_carve(mine, lay.topm, K);  // same region as the list, used before it
   const size_t gw = (size_t)blockIdx.x * kWarps + warp;
   uint32_t* rid = kPath ? ring_ids + gw * kSelectCand : nullptr;
   float* rds = kPath ? ring_dis + gw * kSelectCand : nullptr;
   const uint32_t ep = kPath ? *ep_dev : 0u;
   for (uint32_t b = next_node(ctr, lane); b < n; b = next_node(ctr, lane)) {
     bool tail = false;
-    uint32_t scored = 0;
-    const uint32_t len = collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand,
-                                             cdis, &tail, &scored, lane);
+    collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
+    warp_sort_mark(cand, cdis, lay.L(), lane);
+    const uint32_t len = warp_compact(cand, cdis, lay.L(), b, &tail, lane);
     filter_node(cand, cdis, len, tail, fd, kPath ? 0 : 1, thre, data, norms, dim, k, b, K, nd,
                 P_ids, P_dis, P_cnt, lane);
   }
@@ -1377,7 +1564,7 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   const uint32_t fd = a.final_degree, K = d.k;
   if (!path && K * K < kSelectCand) return fail(TAGORE_EINVAL, "2-hop collect needs K*K >= 480");
   if (path && (a.topm == 0 || a.topm > 256)) return fail(TAGORE_EINVAL, "TOPM must be in [1, 256]");
-  const SelLayout lay{path ? a.topm + K : 0u, kSelectCand + K, 0};
+  const SelLayout lay{path ? a.topm : 0u, K, 0};
   const uint32_t batch = std::min(d.n, kSelectBatch), batches = (d.n + batch - 1) / batch;
   Scratch sc(s);
   // [u64 rows scored][u32 entry point][u32 unused][2 u32 counters per batch] |
@@ -1393,8 +1580,7 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   float* norms = reinterpret_cast<float*>(P_cnt + d.n);
   TG_CUDA(cudaMemsetAsync(work, 0, head, s));
   if (path) {
-    const uint32_t W = a.topm + K;
-    const size_t sm = beam_bytes(W) + 64;
+    const size_t sm = beam_bytes(a.topm, K);
     TG_TRY(set_smem((const void*)k_cal_ep, sm));
     stage_begin("prune_cal_ep", s);
     k_cal_ep<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, K, a.topm, ep_dev);
@@ -1414,10 +1600,10 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   uint32_t* ring_ids = path ? rings.as<uint32_t>() : nullptr;
   float* ring_dis =
       path ? reinterpret_cast<float*>(ring_ids + (size_t)grid * kWarps * kSelectCand) : nullptr;
-  TG_TRY(lists.alloc((size_t)batch * (lay.L * 8 + 4)));
+  TG_TRY(lists.alloc((size_t)batch * (lay.L() * 8 + 4)));
   uint32_t* L_ids = lists.as<uint32_t>();
-  float* L_dis = reinterpret_cast<float*>(L_ids + (size_t)batch * lay.L);
-  uint32_t* L_cnt = reinterpret_cast<uint32_t*>(L_dis + (size_t)batch * lay.L);
+  float* L_dis = reinterpret_cast<float*>(L_ids + (size_t)batch * lay.L());
+  uint32_t* L_cnt = reinterpret_cast<uint32_t*>(L_dis + (size_t)batch * lay.L());
   Scratch ord(s);
   const uint32_t* order = nullptr;
   stage_begin("prune_order", s);
@@ -1440,7 +1626,7 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
     stage_end(sel_name, s);
     TG_CUDA(cudaGetLastError());
     stage_begin("prune_filter", s);
-    k_filter<<<gridf, kWarps * 32, smf, s>>>(L_ids, L_dis, L_cnt, lay.L, d.nd, d.data, norms, first,
+    k_filter<<<gridf, kWarps * 32, smf, s>>>(L_ids, L_dis, L_cnt, lay.L(), d.nd, d.data, norms, first,
                                              cnt, d.dim, K, ctr + 2 * i + 1, fd, path ? 0 : 1,
                                              a.thre, P_ids, P_dis, P_cnt, order);
     count_launch();
@@ -1529,8 +1715,7 @@ int stage_cal_ep(const Dev& d, uint32_t topm, uint32_t* ep_host, cudaStream_t s)
   TG_TRY(validate(d, s));
   Scratch sc(s);
   TG_TRY(sc.alloc(4));
-  const uint32_t W = topm + d.k;
-  const size_t sm = beam_bytes(W) + 64;
+  const size_t sm = beam_bytes(topm, d.k);
   TG_TRY(set_smem((const void*)k_cal_ep, sm));
   k_cal_ep<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, d.k, topm, sc.as<uint32_t>());
   TG_CUDA(cudaGetLastError());
@@ -1603,7 +1788,7 @@ int prune_cfs_static(const Dev& d, const PruneArgs& a, const std::string& mode,
   const size_t tmp = std::max(sort_tmp, scan_tmp);
   // The select kernel's grid is capped here so that its per-warp rings of
   // scored nodes (path collect) stay small: 64 blocks, under 1 MB.
-  SelLayout lay{path ? a.topm + K : 0u, kSelectCand + K, kept_bytes(fd)};
+  SelLayout lay{path ? a.topm : 0u, K, kept_bytes(fd)};
   const size_t sm = lay.bytes() * kWarps;
   const void* fn = path ? (const void*)k_select<true> : (const void*)k_select<false>;
   TG_TRY(set_smem(fn, sm));
@@ -1669,7 +1854,7 @@ int prune_cfs_static(const Dev& d, const PruneArgs& a, const std::string& mode,
   uint32_t* ep_dev = flags + 1;
   uint32_t* ctr = flags + 2;
   if (path) {
-    const size_t sm = beam_bytes(a.topm + K) + 64;
+    const size_t sm = beam_bytes(a.topm, K);
     TG_TRY(set_smem((const void*)k_cal_ep, sm));
     k_cal_ep<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, K, a.topm, ep_dev);
     count_launch();

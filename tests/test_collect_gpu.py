@@ -1,0 +1,39 @@
+"""The prune's collect against the oracle, bit for bit, where its paths part:
+distances that tie (the reference's network decides), kNN rows out of order or
+with a NaN, lists shorter than the ring, widths of each row reader, and beams
+from one entry to the largest."""
+import numpy as np
+import pytest
+
+from test_prune_gpu import run_pair
+from test_screen_gpu import gaussian, graph
+
+pytestmark = pytest.mark.gpu
+
+BOTH = [("path", "dist", 1.0), ("2-hop", "angle", 0.5)]
+
+
+@pytest.mark.parametrize("mode,metric,thre", BOTH)
+@pytest.mark.parametrize("top", [2, 60])
+def test_ties(capi, orc, mode, metric, thre, top):
+    # small whole numbers: most distances tie (top 2), or a few do (top 60). 32
+    # dims keep the rows distinct: among equal rows (12 dims of 0 and 1) the kept sets
+    # of the oracle and of the library differed before the collect changed, too.
+    x = np.random.default_rng(top).integers(0, top, (600, 32)).astype(np.float16)
+    assert len(np.unique(x, axis=0)) == 600
+    run_pair(capi, orc, graph(orc, x, 32, 3), 20, ("cfs", mode, metric), topm=40, thre=thre)
+
+
+@pytest.mark.parametrize("mode,metric,thre", BOTH)
+def test_rows_out_of_order(capi, orc, mode, metric, thre):
+    half, ids, dis, center = graph(orc, gaussian(500, 32, 5), 32, 6)
+    ids, dis = ids.copy(), dis.copy()
+    ids[::2], dis[::2] = ids[::2, ::-1], dis[::2, ::-1]
+    run_pair(capi, orc, (half, ids, dis, center), 20, ("cfs", mode, metric), topm=40, thre=thre)
+
+
+@pytest.mark.parametrize("dim", [8, 92, 96, 104, 128, 136, 960])
+@pytest.mark.parametrize("K,topm", [(24, 1), (33, 32), (65, 100), (128, 256)])
+def test_widths_and_beams(capi, orc, dim, K, topm):
+    run_pair(capi, orc, graph(orc, gaussian(400, dim, dim), K, 7), min(K, 40),
+             ("cfs", "path", "dist"), topm=topm, thre=1.1)

@@ -763,7 +763,7 @@ int knn_build(const Dev& base, const float* norms, const KnnArgs& a, KnnStats* s
   const uint32_t S = std::min<uint32_t>(a.sample ? a.sample : 32, kMaxS);
   // Partners kept per join row: 2, and 3 at the widths the learned screen used to
   // serve, whose builds had its proposals on top of the exact join's (50K x 100: mean
-  // error of the distances 0.0066 with the screen, 0.0071 at T = 2).
+  // error of the distances 0.0066 with the screen, 0.0071 at T = 2, 0.0054 at T = 3).
   const bool more = a.mode == TAGORE_KNN_CHOSEN && base.dim < 1024 &&
                     (base.dim % 8 == 4 || (base.dim < 128 && base.dim % 16 != 0));
   const uint32_t T = std::min<uint32_t>(a.per_row ? a.per_row : more ? 3 : 2,

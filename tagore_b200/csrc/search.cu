@@ -222,8 +222,8 @@ __device__ __forceinline__ void chain4(float& acc, float4 s) {
 }
 
 // Tile of squares (64 dims per row: 4.66 ms, 32: 4.09 ms, by the warps that fit):
-// 32 rows of kUnits 16-byte units, one unit of padding per row so
-// that eight lanes reading a unit each of eight rows meet no bank twice.
+// 32 rows of kUnits 16-byte units, one unit of padding per row so that eight lanes
+// reading a unit each of eight rows meet no bank twice.
 constexpr uint32_t kUnits = 8, kRowFloats = 4 * kUnits + 4;
 constexpr uint32_t kAhead = 4;  // loads in flight per lane
 

@@ -405,9 +405,19 @@ __device__ __noinline__ void warp_sort_mark(uint32_t* cand, float* dis, uint32_t
   __syncwarp();
 }
 
-// Removes the marked entries and the node itself from a sorted, marked list, in
-// place. Returns the entries left; *tail tells whether the list's last entry is
-// among them.
+// The entries of 32 (one per lane, kInv: none) that the filter takes, of a list whose
+// first m were taken before: all but the node itself, which is skipped only until
+// another entry has been taken (:1399-1460). Behind rows equal to its own it is a
+// candidate like any other.
+__device__ __forceinline__ unsigned taken(uint32_t c, uint32_t bid, uint32_t m) {
+  const unsigned any = __ballot_sync(kFull, c != kInv);
+  const unsigned other = __ballot_sync(kFull, c != kInv && c != bid);
+  return m ? any : any & ~((other & (0u - other)) - 1u);
+}
+
+// Removes the marked entries and the node itself where it is skipped (taken) from a
+// sorted, marked list, in place. Returns the entries left; *tail tells whether the
+// list's last entry is among them.
 __device__ __forceinline__ uint32_t warp_compact(uint32_t* cand, float* dis, uint32_t len, uint32_t bid,
                                  bool* tail, int lane) {
   const unsigned below = (1u << lane) - 1u;
@@ -417,9 +427,9 @@ __device__ __forceinline__ uint32_t warp_compact(uint32_t* cand, float* dis, uin
     const uint32_t i = base + lane;
     const uint32_t c = i < len ? cand[i] : kInv;
     const float d = i < len ? dis[i] : 0.0f;
-    ok = __ballot_sync(kFull, c != kInv && c != bid);
+    ok = taken(c, bid, m);
     __syncwarp();  // the chunk is read before an earlier or equal place is written
-    if (c != kInv && c != bid) {
+    if ((ok >> lane) & 1u) {
       const uint32_t p = m + __popc(ok & below);
       cand[p] = c;
       dis[p] = d;
@@ -580,9 +590,9 @@ __device__ __noinline__ int warp_list(uint32_t* cand, float* cdis, uint32_t* mar
     uint32_t prev = __shfl_up_sync(kFull, c, 1);
     if (lane == 0) prev = carry;
     carry = __shfl_sync(kFull, c, 31);
-    const bool keep = c != kInv && c != bid && !(f >= 1 && c == prev);
-    ok = __ballot_sync(kFull, keep);
-    if (keep) {
+    if (f >= 1 && c == prev) c = kInv;
+    ok = taken(c, bid, m);
+    if ((ok >> lane) & 1u) {
       const uint32_t p = m + __popc(ok & below);
       out_ids[p] = c;
       out_dis[p] = d;

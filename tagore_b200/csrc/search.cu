@@ -347,7 +347,9 @@ struct WarpSearch {
     __syncwarp();
     // lane i < m holds the batch's i-th new entry from here on
     const uint32_t mine = lane < m ? row_id[lane] : kNone;
-    const float d = score(m);
+    // A NaN ranks as infinite: the places below need an order of all distances, or
+    // two entries take one place and another keeps a stale id.
+    const float d = fminf(score(m), INFINITY);
     // with a full pool, one no closer than its last entry changes nothing
     const uint32_t L = a.L;
     const bool enter = lane < m && !(size == L && P[L - 1].d <= d);

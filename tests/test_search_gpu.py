@@ -115,3 +115,22 @@ def test_rejects_bad_arguments(capi):
         capi.search(base, offs, adj, 10, base[:2].contiguous(), 8, 3)   # entry point outside
     with pytest.raises(capi.TagoreError):
         capi.search(base, offs, adj, 0, base[:2].contiguous(), 0, 3)    # empty pool
+
+
+@pytest.mark.parametrize("seed", [0, 21])
+def test_nan_distances_rank_as_infinite(capi, orc, seed):
+    # NaN in rows of the base (every eighth), and in a whole query: the oracle takes
+    # infinities, which give those distances without a NaN
+    rng = np.random.default_rng(12)
+    base = rng.integers(0, 200, (4000, 20)).astype(np.float32)
+    queries = rng.integers(0, 200, (40, 20)).astype(np.float32)
+    offs, adj = ragged_graph(4000, 30, rng)
+    nan, inf = base.copy(), base.copy()
+    nan[::8, 3], inf[::8, 3] = np.nan, np.inf
+    for L in (40, 200):
+        got, _ = both(capi, orc, nan, offs, adj, 17, queries, L, 20, seed)
+        assert np.array_equal(got, orc.greedy_search(inf, offs, adj, 17, queries, L, 20, seed))
+        q_nan, q_inf = queries.copy(), queries.copy()
+        q_nan[::2, 5], q_inf[::2, 5] = np.nan, np.inf
+        got, _ = both(capi, orc, base, offs, adj, 17, q_nan, L, 20, seed)
+        assert np.array_equal(got, orc.greedy_search(base, offs, adj, 17, q_inf, L, 20, seed))

@@ -415,11 +415,13 @@ __device__ __forceinline__ unsigned taken(uint32_t c, uint32_t bid, uint32_t m) 
   return m ? any : any & ~((other & (0u - other)) - 1u);
 }
 
+// The length of a compacted list, with this bit where the list's last entry is left.
+constexpr uint32_t kTailBit = 0x80000000u;
+
 // Removes the marked entries and the node itself where it is skipped (taken) from a
-// sorted, marked list, in place. Returns the entries left; *tail tells whether the
-// list's last entry is among them.
-__device__ __forceinline__ uint32_t warp_compact(uint32_t* cand, float* dis, uint32_t len, uint32_t bid,
-                                 bool* tail, int lane) {
+// sorted, marked list, in place. Returns the entries left and the tail bit.
+__device__ __noinline__ uint32_t warp_compact(uint32_t* cand, float* dis, uint32_t len,
+                                              uint32_t bid, int lane) {
   const unsigned below = (1u << lane) - 1u;
   uint32_t m = 0;
   unsigned ok = 0;
@@ -437,8 +439,7 @@ __device__ __forceinline__ uint32_t warp_compact(uint32_t* cand, float* dis, uin
     m += __popc(ok);
   }
   __syncwarp();
-  *tail = len > 0 && ((ok >> ((len - 1) & 31u)) & 1u);
-  return m;
+  return len > 0 && ((ok >> ((len - 1) & 31u)) & 1u) ? m | kTailBit : m;
 }
 
 // Words that mark the places of the kNN row's entries in the merged list.
@@ -448,7 +449,7 @@ constexpr uint32_t kMarkWords = (kSelectCand + 128 + 31) / 32;
 // kSelectCand collected ones, in shared memory) where the order of equal
 // distances cannot be observed, written to out_ids / out_dis: the collected
 // entries are sorted in registers and merged with the row, which is sorted
-// already. Returns the entries left, or -1 where the network has to decide: a
+// already. Returns as warp_compact does, or kInv where the network has to decide: a
 // row out of order, a distance that is negative or NaN, or equal distances of
 // different ids (entries with the same id and distance are the same in any
 // order). The collected part of the list is overwritten.
@@ -458,9 +459,10 @@ constexpr uint32_t kMarkWords = (kSelectCand + 128 + 31) / 32;
 // of the 45 passes exchange within a lane; every merge starts mirrored, which
 // leaves one direction of comparison.
 // Collect at 500K x 96, K = 64: 29.1 ms with the network, 28.0 ms with this.
-__device__ __noinline__ int warp_list(uint32_t* cand, float* cdis, uint32_t* mark, uint32_t K,
-                                      uint32_t bid, uint32_t* __restrict__ out_ids,
-                                      float* __restrict__ out_dis, bool* tail, int lane) {
+__device__ __noinline__ uint32_t warp_list(uint32_t* cand, float* cdis, uint32_t* mark,
+                                           uint32_t K, uint32_t bid,
+                                           uint32_t* __restrict__ out_ids,
+                                           float* __restrict__ out_dis, int lane) {
   constexpr uint32_t kLast = 0x7F800000u;  // bits of +inf
   constexpr int E = 16;
   static_assert(kSelectCand == 30 * E, "the pads fill the last two lanes");
@@ -483,7 +485,7 @@ __device__ __noinline__ int warp_list(uint32_t* cand, float* cdis, uint32_t* mar
       bad |= k < p || (k == p && cand[i] != cand[i - 1]);
     }
   }
-  if (__any_sync(kFull, bad)) return -1;
+  if (__any_sync(kFull, bad)) return kInv;
   // ascending, position 16 * lane + t
   auto in_lane = [&](int a, int b) {
     const bool s = key[a] > key[b];
@@ -544,7 +546,7 @@ __device__ __noinline__ int warp_list(uint32_t* cand, float* cdis, uint32_t* mar
     const uint32_t nk = __shfl_down_sync(kFull, key[0], 1), ni = __shfl_down_sync(kFull, id[0], 1);
     bad |= lane < 31 && key[E - 1] == nk && id[E - 1] != ni;
   }
-  if (__any_sync(kFull, bad)) return -1;
+  if (__any_sync(kFull, bad)) return kInv;
   // back to the list, the 16 places of a lane permuted against bank conflicts
   auto place = [](uint32_t p) { return (p & ~15u) | ((p ^ (p >> 4)) & 15u); };
   if (lane < 30) {
@@ -572,7 +574,7 @@ __device__ __noinline__ int warp_list(uint32_t* cand, float* cdis, uint32_t* mar
     const uint32_t f = i + lo;
     atomicOr(&mark[f >> 5], 1u << (f & 31u));
   }
-  if (__any_sync(kFull, bad)) return -1;
+  if (__any_sync(kFull, bad)) return kInv;
   __syncwarp();
   const unsigned below = (1u << lane) - 1u;
   const uint32_t total = K + kSelectCand;
@@ -600,8 +602,7 @@ __device__ __noinline__ int warp_list(uint32_t* cand, float* cdis, uint32_t* mar
     m += __popc(ok);
     rows += __popc(w);
   }
-  *tail = (ok >> ((total - 1) & 31u)) & 1u;
-  return (int)m;
+  return (ok >> ((total - 1) & 31u)) & 1u ? m | kTailBit : m;
 }
 
 // Kept neighbours of one node, and the rows of a tile that outlived the kept
@@ -890,8 +891,36 @@ __device__ __forceinline__ void filter_node(const uint32_t* cand, const float* c
   __syncwarp();
 }
 
+// The list as it was collected, sorted by the network: where warp_list cannot decide.
+// Out of line, so that it takes no registers of the collect, which spills at its
+// seven blocks per SM (1M x 128: 82.3 ms inlined, 79.5 ms; six blocks 81.0 ms).
+template <bool kPath>
+static __device__ __noinline__ uint32_t network_list(const uint32_t* __restrict__ G, uint32_t K,
+                                                     uint32_t scored, const uint32_t* rid,
+                                                     const float* rds, uint32_t* cand, float* cdis,
+                                                     uint32_t b, uint32_t* __restrict__ out_ids,
+                                                     float* out_dis, int lane) {
+  for (uint32_t j = lane; j < kSelectCand; j += 32) {
+    if (kPath) {
+      cand[K + j] = j < scored ? rid[j] : kInv;
+      cdis[K + j] = j < scored ? rds[j] : kInfDis;
+    } else {
+      cand[K + j] = __ldg(G + (size_t)cand[j / K] * K + j % K);
+      cdis[K + j] = out_dis[j];
+    }
+  }
+  __syncwarp();
+  warp_sort_mark(cand, cdis, kSelectCand + K, lane);
+  const uint32_t got = warp_compact(cand, cdis, kSelectCand + K, b, lane);
+  for (uint32_t j = lane; j < (got & ~kTailBit); j += 32) {
+    out_ids[j] = cand[j];
+    out_dis[j] = cdis[j];
+  }
+  return got;
+}
+
 // Candidate lists of the nodes at positions [first, first + cnt) of the order,
-// L entries apart; L_cnt holds a list's length and, in its top bit, `tail`.
+// L entries apart; L_cnt holds a list's length and its tail bit.
 // ring_ids / ring_dis: per-warp rings of kSelectCand scored nodes (path), by the
 // warp's global number.
 //
@@ -899,8 +928,6 @@ __device__ __forceinline__ void filter_node(const uint32_t* cand, const float* c
 // (about 4 KB written and read per node, 1.4 ms of a 1M prune): the beam waits on
 // gathers and wants warps, the filter's tiles want registers, and each half's
 // code fits the instruction cache.
-constexpr uint32_t kTailBit = 0x80000000u;
-
 template <bool kPath>
 __global__ void __launch_bounds__(kWarps * 32, 7)
     k_collect(const uint32_t* __restrict__ G, const float* __restrict__ nd,
@@ -925,7 +952,6 @@ __global__ void __launch_bounds__(kWarps * 32, 7)
   unsigned long long rows = 0;
   for (uint32_t i = next_node(ctr, lane); i < cnt; i = next_node(ctr, lane)) {
     const uint32_t b = node_at(order, first + i);
-    bool tail = false;
     const uint32_t scored =
         collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
     uint32_t* out_ids = L_ids + (size_t)i * lay.L();
@@ -935,29 +961,11 @@ __global__ void __launch_bounds__(kWarps * 32, 7)
       for (uint32_t j = lane; j < kSelectCand; j += 32) out_dis[j] = cdis[K + j];
       __syncwarp();
     }
-    int got = warp_list(cand, cdis, mark, K, b, out_ids, out_dis, &tail, lane);
-    if (got < 0) {
-      // the list as it was collected, sorted by the network
-      for (uint32_t j = lane; j < kSelectCand; j += 32) {
-        if (kPath) {
-          cand[K + j] = j < scored ? rid[j] : kInv;
-          cdis[K + j] = j < scored ? rds[j] : kInfDis;
-        } else {
-          cand[K + j] = __ldg(G + (size_t)cand[j / K] * K + j % K);
-          cdis[K + j] = out_dis[j];
-        }
-      }
-      __syncwarp();
-      warp_sort_mark(cand, cdis, lay.L(), lane);
-      got = (int)warp_compact(cand, cdis, lay.L(), b, &tail, lane);
-      for (uint32_t j = lane; j < (uint32_t)got; j += 32) {
-        out_ids[j] = cand[j];
-        out_dis[j] = cdis[j];
-      }
-    }
-    const uint32_t len = (uint32_t)got;
-    rows += scored + len;
-    if (lane == 0) L_cnt[i] = len | (tail ? kTailBit : 0u);
+    uint32_t got = warp_list(cand, cdis, mark, K, b, out_ids, out_dis, lane);
+    if (got == kInv)
+      got = network_list<kPath>(G, K, scored, rid, rds, cand, cdis, b, out_ids, out_dis, lane);
+    rows += scored + (got & ~kTailBit);
+    if (lane == 0) L_cnt[i] = got;
     __syncwarp();
   }
   if (work && lane == 0) atomicAdd(work, rows);
@@ -1003,12 +1011,11 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   float* rds = kPath ? ring_dis + gw * kSelectCand : nullptr;
   const uint32_t ep = kPath ? *ep_dev : 0u;
   for (uint32_t b = next_node(ctr, lane); b < n; b = next_node(ctr, lane)) {
-    bool tail = false;
     collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
     warp_sort_mark(cand, cdis, lay.L(), lane);
-    const uint32_t len = warp_compact(cand, cdis, lay.L(), b, &tail, lane);
-    filter_node(cand, cdis, len, tail, fd, kPath ? 0 : 1, thre, data, norms, dim, k, b, K, nd,
-                P_ids, P_dis, P_cnt, lane);
+    const uint32_t len = warp_compact(cand, cdis, lay.L(), b, lane);
+    filter_node(cand, cdis, len & ~kTailBit, (len & kTailBit) != 0, fd, kPath ? 0 : 1, thre, data,
+                norms, dim, k, b, K, nd, P_ids, P_dis, P_cnt, lane);
   }
 }
 
@@ -1069,9 +1076,9 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
     uint32_t out_cnt;
     if (len > fd) {
       warp_sort_mark(cand, cdis, len, lane);
-      bool tail = false;
-      const uint32_t left = warp_compact(cand, cdis, len, b, &tail, lane);
-      out_cnt = warp_filter(cand, cdis, left, tail, fd, metric, thre, data, norms, dim, k, lane);
+      const uint32_t left = warp_compact(cand, cdis, len, b, lane);
+      out_cnt = warp_filter(cand, cdis, left & ~kTailBit, (left & kTailBit) != 0, fd, metric, thre,
+                            data, norms, dim, k, lane);
     } else {
       // Union in ascending reverse-slot order (:1632-1647).
       for (uint32_t i = lane; i < cur_num; i += 32) sel[i] = cand[i];

@@ -303,6 +303,12 @@ __device__ __forceinline__ float row_dist128(const __half* __restrict__ a,
   return dist128_pairs([&](int p, int w) { return __ldg((w ? B : A) + p); });
 }
 
+// Whether rows of `dim` halves (a multiple of 4) from `p` on may be read 16 bytes at
+// a time. A caller's buffers may start on any 8 bytes.
+__device__ __forceinline__ bool rows_of_16(const __half* p, uint32_t dim) {
+  return (dim & 7u) == 0 && ((uintptr_t)p & 15u) == 0;
+}
+
 // The same distance between two FP16 rows of `dim` halves (a multiple of 4)
 // by a single thread, so that the 32 lanes of a warp score 32 rows at once.
 // Kept out of line: one copy of the unrolled tree serves every call site and
@@ -311,16 +317,12 @@ static __device__ __noinline__ float row_dist(const __half* __restrict__ a,
                                               const __half* __restrict__ b, uint32_t dim) {
   const uint2* A = reinterpret_cast<const uint2*>(a);
   const uint2* B = reinterpret_cast<const uint2*>(b);
-  if (dim == 128) return row_dist128(a, b);
-  if (dim == 96) {
+  if (rows_of_16(a, dim) && rows_of_16(b, dim)) {
+    if (dim == 128) return row_dist128(a, b);
     const uint4* A4 = reinterpret_cast<const uint4*>(a);
     const uint4* B4 = reinterpret_cast<const uint4*>(b);
-    return dist_pairs_fixed<12>([&](uint32_t u, int w) { return __ldg((w ? B4 : A4) + u); });
-  }
-  if ((dim & 7u) == 0) {
-    const uint4* A4 = reinterpret_cast<const uint4*>(a);
-    const uint4* B4 = reinterpret_cast<const uint4*>(b);
-    return dist_pairs_rounds([&](uint32_t u, int w) { return __ldg((w ? B4 : A4) + u); }, dim >> 3);
+    auto load = [&](uint32_t u, int w) { return __ldg((w ? B4 : A4) + u); };
+    return dim == 96 ? dist_pairs_fixed<12>(load) : dist_pairs_rounds(load, dim >> 3);
   }
   const uint32_t chunks = dim >> 2;
   auto leaf = [&](int slot, float& x, float& y) {
@@ -434,12 +436,13 @@ __device__ __forceinline__ float warp_rows32_fixed(const __half* q, const __half
 }
 
 // Any width that is a multiple of four, 16 rows at a time.
+template <bool kWide>
 static __device__ __noinline__ float warp_rows32_any(const __half* q,
                                                      const __half* __restrict__ base, uint32_t dim,
                                                      const uint32_t* ids, uint32_t m) {
   const uint32_t lane = threadIdx.x & 31u, g = lane >> 2, j = lane & 3u;
   const uint32_t chunks = dim >> 2, units = (dim + 7) >> 3;
-  const bool aligned = (dim & 7u) == 0;
+  const bool aligned = kWide && (dim & 7u) == 0;
   auto unit = [&](const __half* row, uint32_t u) {
     if (aligned) return __ldg(reinterpret_cast<const uint4*>(row) + u);
     const uint2* r = reinterpret_cast<const uint2*>(row);
@@ -493,11 +496,17 @@ static __device__ __noinline__ float warp_rows32_any(const __half* q,
   return j < 2 ? lo : hi;
 }
 
+// kWide: rows and query may be read 16 bytes at a time where the width allows it. At
+// compile time: a flag carried through the collect costs it 2.6 ms of spills (79.7 ->
+// 82.3 ms at 1M x 128).
+template <bool kWide>
 __device__ __forceinline__ float warp_rows32(const __half* q, const __half* __restrict__ base,
                                              uint32_t dim, const uint32_t* ids, uint32_t m) {
-  if (dim == 128) return warp_rows32_fixed<128>(q, base, ids, m);
-  if (dim == 96) return warp_rows32_fixed<96>(q, base, ids, m);
-  return warp_rows32_any(q, base, dim, ids, m);
+  if constexpr (kWide) {
+    if (dim == 128) return warp_rows32_fixed<128>(q, base, ids, m);
+    if (dim == 96) return warp_rows32_fixed<96>(q, base, ids, m);
+  }
+  return warp_rows32_any<kWide>(q, base, dim, ids, m);
 }
 
 // distance_filter (src/Tagore_src.cu:1488-1490) as nvcc compiles it, one fused

@@ -249,6 +249,8 @@ __device__ __noinline__ void beam_update(Beam bm, uint32_t topm, uint32_t K, con
   if (!ok) beam_network(bm, 0, W, lane);
 }
 
+// kWide: as warp_rows32's.
+template <bool kWide>
 __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __restrict__ data,
                               uint32_t dim, uint32_t K, const __half* query, uint32_t start,
                               uint32_t topm, uint32_t iters, Beam bm, uint32_t* ring_id,
@@ -308,7 +310,7 @@ __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __re
     __syncwarp();
     for (uint32_t base = 0; base < nfresh; base += 32) {
       const uint32_t r = base + own;
-      const float d = warp_rows32(query, data, dim, bm.sid + base, min(32u, nfresh - base));
+      const float d = warp_rows32<kWide>(query, data, dim, bm.sid + base, min(32u, nfresh - base));
       if (r < nfresh) {
         bm.dis[topm + fresh_at[r]] = d;
         if (ring_id) {
@@ -793,6 +795,7 @@ __global__ void k_validate(const uint32_t* __restrict__ g, size_t cnt, uint32_t 
 }
 
 // cal_ep_gpu (:1889-2058): one warp, 30 expansions from node 0 toward the centre.
+template <bool kWide>
 __global__ void k_cal_ep(const uint32_t* __restrict__ G, const __half* __restrict__ data,
                          const __half* __restrict__ center, uint32_t dim, uint32_t K,
                          uint32_t topm, uint32_t* ep) {
@@ -800,8 +803,8 @@ __global__ void k_cal_ep(const uint32_t* __restrict__ G, const __half* __restric
   Beam bm = beam_carve(smem, topm, K);
   const int lane = threadIdx.x & 31;
   if (threadIdx.x >= 32) return;
-  const uint32_t best = warp_beam(G, data, dim, K, center, 0, topm, 30, bm, nullptr, nullptr,
-                                  nullptr, lane);
+  const uint32_t best = warp_beam<kWide>(G, data, dim, K, center, 0, topm, 30, bm, nullptr, nullptr,
+                                         nullptr, lane);
   if (lane == 0) *ep = best;
 }
 
@@ -821,7 +824,7 @@ __device__ __forceinline__ uint32_t node_at(const uint32_t* __restrict__ order, 
 // node b's candidates (its kNN row and the collected nodes), unsorted, in
 // cand / cdis. Returns the rows scored. rid / rds: this warp's ring of kSelectCand
 // scored nodes (path).
-template <bool kPath>
+template <bool kPath, bool kWide>
 __device__ __forceinline__ uint32_t collect_node(
     const uint32_t* __restrict__ G, const float* __restrict__ nd, const __half* __restrict__ data,
     uint32_t dim, uint32_t K, uint32_t ep, uint32_t topm, uint32_t b, Beam bm, uint32_t* rid,
@@ -830,7 +833,7 @@ __device__ __forceinline__ uint32_t collect_node(
   uint32_t scored = kSelectCand;  // 2-hop: the 480 collected
   if (kPath) {
     uint32_t curr = 0;
-    warp_beam(G, data, dim, K, q, ep, topm, 10, bm, rid, rds, &curr, lane);
+    warp_beam<kWide>(G, data, dim, K, q, ep, topm, 10, bm, rid, rds, &curr, lane);
     scored = curr;
     __syncwarp();  // the ring (global) and the beam's region are done
     for (uint32_t i = lane; i < kSelectCand; i += 32) {
@@ -928,7 +931,7 @@ static __device__ __noinline__ uint32_t network_list(const uint32_t* __restrict_
 // (about 4 KB written and read per node, 1.4 ms of a 1M prune): the beam waits on
 // gathers and wants warps, the filter's tiles want registers, and each half's
 // code fits the instruction cache.
-template <bool kPath>
+template <bool kPath, bool kWide>
 __global__ void __launch_bounds__(kWarps * 32, 7)
     k_collect(const uint32_t* __restrict__ G, const float* __restrict__ nd,
               const __half* __restrict__ data, uint32_t first, uint32_t cnt, uint32_t dim,
@@ -953,7 +956,7 @@ __global__ void __launch_bounds__(kWarps * 32, 7)
   for (uint32_t i = next_node(ctr, lane); i < cnt; i = next_node(ctr, lane)) {
     const uint32_t b = node_at(order, first + i);
     const uint32_t scored =
-        collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
+        collect_node<kPath, kWide>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
     uint32_t* out_ids = L_ids + (size_t)i * lay.L();
     float* out_dis = L_dis + (size_t)i * lay.L();
     if (!kPath) {
@@ -990,7 +993,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 
 // Both halves by the same warp, the list in shared memory: for the prune that
 // may not allocate the lists.
-template <bool kPath>
+template <bool kPath, bool kWide>
 __global__ void __launch_bounds__(kWarps * 32, 4)
     k_select(const uint32_t* __restrict__ G, float* __restrict__ nd, const __half* __restrict__ data,
              const float* __restrict__ norms, uint32_t n, uint32_t dim, uint32_t K,
@@ -1011,7 +1014,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   float* rds = kPath ? ring_dis + gw * kSelectCand : nullptr;
   const uint32_t ep = kPath ? *ep_dev : 0u;
   for (uint32_t b = next_node(ctr, lane); b < n; b = next_node(ctr, lane)) {
-    collect_node<kPath>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
+    collect_node<kPath, kWide>(G, nd, data, dim, K, ep, topm, b, bm, rid, rds, cand, cdis, lane);
     warp_sort_mark(cand, cdis, lay.L(), lane);
     const uint32_t len = warp_compact(cand, cdis, lay.L(), b, lane);
     filter_node(cand, cdis, len & ~kTailBit, (len & kTailBit) != 0, fd, kPath ? 0 : 1, thre, data,
@@ -1557,6 +1560,18 @@ int reverse_grid(uint32_t fd, uint32_t K, uint32_t n, int* grid) {
 // 1.2 GB at K = 96) and still fills the chip hundreds of times over.
 constexpr uint32_t kSelectBatch = 1u << 18;
 
+bool on_16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+int launch_cal_ep(const Dev& d, uint32_t topm, uint32_t* ep_dev, cudaStream_t s) {
+  auto* fn = on_16(d.data) && on_16(d.center) ? k_cal_ep<true> : k_cal_ep<false>;
+  const size_t sm = beam_bytes(topm, d.k);
+  TG_TRY(set_smem((const void*)fn, sm));
+  fn<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, d.k, topm, ep_dev);
+  count_launch();
+  TG_CUDA(cudaGetLastError());
+  return TAGORE_OK;
+}
+
 void launch_row_norms(const Dev& d, float* norms, cudaStream_t s) {
   k_row_norms<<<grid_for(8, d.n), 256, 0, s>>>(d.data, d.n, d.dim, norms);
   count_launch();
@@ -1597,20 +1612,18 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   float* norms = reinterpret_cast<float*>(P_cnt + d.n);
   TG_CUDA(cudaMemsetAsync(work, 0, head, s));
   if (path) {
-    const size_t sm = beam_bytes(a.topm, K);
-    TG_TRY(set_smem((const void*)k_cal_ep, sm));
     stage_begin("prune_cal_ep", s);
-    k_cal_ep<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, K, a.topm, ep_dev);
-    count_launch();
+    TG_TRY(launch_cal_ep(d, a.topm, ep_dev, s));
     stage_end("prune_cal_ep", s);
-    TG_CUDA(cudaGetLastError());
   }
   const size_t sm = lay.bytes() * kWarps, smf = kept_bytes(fd) * kWarps;
-  const void* fn = path ? (const void*)k_collect<true> : (const void*)k_collect<false>;
-  TG_TRY(set_smem(fn, sm));
+  auto* fn = !path           ? k_collect<false, true>
+             : on_16(d.data) ? k_collect<true, true>
+                             : k_collect<true, false>;
+  TG_TRY(set_smem((const void*)fn, sm));
   TG_TRY(set_smem((const void*)k_filter, smf));
   int grid = 0, gridf = 0;
-  TG_TRY(resident_grid(fn, kWarps * 32, sm, kWarps, batch, &grid));
+  TG_TRY(resident_grid((const void*)fn, kWarps * 32, sm, kWarps, batch, &grid));
   TG_TRY(resident_grid((const void*)k_filter, kWarps * 32, smf, kWarps, batch, &gridf));
   Scratch rings(s), lists(s);
   if (path) TG_TRY(rings.alloc((size_t)grid * kWarps * kSelectCand * 8));
@@ -1631,14 +1644,9 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   for (uint32_t i = 0; i < batches; ++i) {
     const uint32_t first = i * batch, cnt = std::min(batch, d.n - first);
     stage_begin(sel_name, s);
-    if (path)
-      k_collect<true><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, first, cnt, d.dim, K,
-                                                    ep_dev, ctr + 2 * i, a.topm, L_ids, L_dis,
-                                                    L_cnt, work, ring_ids, ring_dis, order);
-    else
-      k_collect<false><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, first, cnt, d.dim, K,
-                                                     ep_dev, ctr + 2 * i, a.topm, L_ids, L_dis,
-                                                     L_cnt, work, nullptr, nullptr, order);
+    fn<<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, first, cnt, d.dim, K, ep_dev,
+                                     ctr + 2 * i, a.topm, L_ids, L_dis, L_cnt, work, ring_ids,
+                                     ring_dis, order);
     count_launch();
     stage_end(sel_name, s);
     TG_CUDA(cudaGetLastError());
@@ -1732,10 +1740,7 @@ int stage_cal_ep(const Dev& d, uint32_t topm, uint32_t* ep_host, cudaStream_t s)
   TG_TRY(validate(d, s));
   Scratch sc(s);
   TG_TRY(sc.alloc(4));
-  const size_t sm = beam_bytes(topm, d.k);
-  TG_TRY(set_smem((const void*)k_cal_ep, sm));
-  k_cal_ep<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, d.k, topm, sc.as<uint32_t>());
-  TG_CUDA(cudaGetLastError());
+  TG_TRY(launch_cal_ep(d, topm, sc.as<uint32_t>(), s));
   TG_CUDA(cudaMemcpyAsync(ep_host, sc.p, 4, cudaMemcpyDeviceToHost, s));
   TG_CUDA(cudaStreamSynchronize(s));
   return TAGORE_OK;
@@ -1807,10 +1812,12 @@ int prune_cfs_static(const Dev& d, const PruneArgs& a, const std::string& mode,
   // scored nodes (path collect) stay small: 64 blocks, under 1 MB.
   SelLayout lay{path ? a.topm : 0u, K, kept_bytes(fd)};
   const size_t sm = lay.bytes() * kWarps;
-  const void* fn = path ? (const void*)k_select<true> : (const void*)k_select<false>;
-  TG_TRY(set_smem(fn, sm));
+  auto* fn = !path           ? k_select<false, true>
+             : on_16(d.data) ? k_select<true, true>
+                             : k_select<true, false>;
+  TG_TRY(set_smem((const void*)fn, sm));
   int grid = 0;
-  TG_TRY(resident_grid(fn, kWarps * 32, sm, kWarps, d.n, &grid));
+  TG_TRY(resident_grid((const void*)fn, kWarps * 32, sm, kWarps, d.n, &grid));
   grid = std::min(grid, 64);
   const size_t ring_n = path ? (size_t)grid * kWarps * kSelectCand : 0;
   // Layout: flags | select rows | reverse-edge keys | CUB temporary | rings.
@@ -1870,26 +1877,14 @@ int prune_cfs_static(const Dev& d, const PruneArgs& a, const std::string& mode,
   // select (as run_dist_prune)
   uint32_t* ep_dev = flags + 1;
   uint32_t* ctr = flags + 2;
-  if (path) {
-    const size_t sm = beam_bytes(a.topm, K);
-    TG_TRY(set_smem((const void*)k_cal_ep, sm));
-    k_cal_ep<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, K, a.topm, ep_dev);
-    count_launch();
-    TG_CUDA(cudaGetLastError());
-  }
+  if (path) TG_TRY(launch_cal_ep(d, a.topm, ep_dev, s));
   // The screens' norms take the place of the reverse-edge keys (E >= n words),
   // which are written after the select and read before filter_reverse.
   float* norms = reinterpret_cast<float*>(keys);
   launch_row_norms(d, norms, s);
   TG_CUDA(cudaGetLastError());
-  if (path)
-    k_select<true><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, norms, d.n, d.dim, K,
-                                                 ep_dev, ctr, a.topm, fd, a.thre, P_ids, P_dis,
-                                                 P_cnt, ring_ids, ring_dis);
-  else
-    k_select<false><<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, norms, d.n, d.dim, K,
-                                                  ep_dev, ctr, a.topm, fd, a.thre, P_ids, P_dis,
-                                                  P_cnt, nullptr, nullptr);
+  fn<<<grid, kWarps * 32, sm, s>>>(d.graph, d.nd, d.data, norms, d.n, d.dim, K, ep_dev, ctr, a.topm,
+                                   fd, a.thre, P_ids, P_dis, P_cnt, ring_ids, ring_dis);
   count_launch();
   TG_CUDA(cudaGetLastError());
 

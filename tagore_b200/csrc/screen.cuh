@@ -192,7 +192,7 @@ __device__ __forceinline__ uint2 screen_rows(const __half* __restrict__ data, ui
                                              const ScreenRule& rule, uint32_t id, float nr,
                                              float dis, const uint32_t* bid, const float* bn,
                                              const float* bd, uint32_t nb, float* tile) {
-  if ((dim & 7u) == 0)
+  if (rows_of_16(data, dim))
     return screen_tile<true, kAny>(data, dim, rule, id, nr, dis, bid, bn, bd, nb, tile);
   return screen_tile<false, kAny>(data, dim, rule, id, nr, dis, bid, bn, bd, nb, tile);
 }

@@ -146,6 +146,7 @@ int pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();  // a caller that goes on with less must not meet it again
     return cuda_fail(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
   }
   return TAGORE_OK;

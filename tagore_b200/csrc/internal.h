@@ -79,9 +79,11 @@ struct Scratch {
   }
   template <class T>
   T* as() const { return reinterpret_cast<T*>(p); }
-  ~Scratch() {
+  void release() {
     if (p) pool_free(p, s);
+    p = nullptr;
   }
+  ~Scratch() { release(); }
   Scratch(const Scratch&) = delete;
   Scratch& operator=(const Scratch&) = delete;
 };

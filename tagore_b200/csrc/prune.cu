@@ -1557,8 +1557,9 @@ int reverse_grid(uint32_t fd, uint32_t K, uint32_t n, int* grid) {
 }
 
 // Nodes per collect / filter pair: bounds the candidate lists in memory (about
-// 1.2 GB at K = 96) and still fills the chip hundreds of times over.
-constexpr uint32_t kSelectBatch = 1u << 18;
+// 1.2 GB at K = 96) and still fills the chip dozens of times over. Where the device
+// has no room for them the batch is halved, down to kMinBatch (under 3 MB).
+constexpr uint32_t kSelectBatch = 1u << 18, kMinBatch = 1u << 9;
 
 bool on_16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
@@ -1597,15 +1598,12 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   if (!path && K * K < kSelectCand) return fail(TAGORE_EINVAL, "2-hop collect needs K*K >= 480");
   if (path && (a.topm == 0 || a.topm > 256)) return fail(TAGORE_EINVAL, "TOPM must be in [1, 256]");
   const SelLayout lay{path ? a.topm : 0u, K, 0};
-  const uint32_t batch = std::min(d.n, kSelectBatch), batches = (d.n + batch - 1) / batch;
   Scratch sc(s);
-  // [u64 rows scored][u32 entry point][u32 unused][2 u32 counters per batch] |
-  // select rows | norms
-  const size_t head = 16 + (((size_t)batches * 8 + 15) & ~(size_t)15);
+  // [u64 rows scored][u32 entry point][u32 unused] | select rows | norms
+  const size_t head = 16;
   TG_TRY(sc.alloc(head + (size_t)d.n * fd * 8 + (size_t)d.n * 8));
   unsigned long long* work = sc.as<unsigned long long>();
   uint32_t* ep_dev = reinterpret_cast<uint32_t*>(work + 1);
-  uint32_t* ctr = ep_dev + 2;
   uint32_t* P_ids = reinterpret_cast<uint32_t*>(sc.as<unsigned char>() + head);
   float* P_dis = reinterpret_cast<float*>(P_ids + (size_t)d.n * fd);
   uint32_t* P_cnt = reinterpret_cast<uint32_t*>(P_dis + (size_t)d.n * fd);
@@ -1623,23 +1621,33 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   TG_TRY(set_smem((const void*)fn, sm));
   TG_TRY(set_smem((const void*)k_filter, smf));
   int grid = 0, gridf = 0;
-  TG_TRY(resident_grid((const void*)fn, kWarps * 32, sm, kWarps, batch, &grid));
-  TG_TRY(resident_grid((const void*)k_filter, kWarps * 32, smf, kWarps, batch, &gridf));
+  TG_TRY(resident_grid((const void*)fn, kWarps * 32, sm, kWarps, d.n, &grid));
+  TG_TRY(resident_grid((const void*)k_filter, kWarps * 32, smf, kWarps, d.n, &gridf));
   Scratch rings(s), lists(s);
   if (path) TG_TRY(rings.alloc((size_t)grid * kWarps * kSelectCand * 8));
   uint32_t* ring_ids = path ? rings.as<uint32_t>() : nullptr;
   float* ring_dis =
       path ? reinterpret_cast<float*>(ring_ids + (size_t)grid * kWarps * kSelectCand) : nullptr;
-  TG_TRY(lists.alloc((size_t)batch * (lay.L() * 8 + 4)));
-  uint32_t* L_ids = lists.as<uint32_t>();
-  float* L_dis = reinterpret_cast<float*>(L_ids + (size_t)batch * lay.L());
-  uint32_t* L_cnt = reinterpret_cast<uint32_t*>(L_dis + (size_t)batch * lay.L());
   Scratch ord(s);
   const uint32_t* order = nullptr;
   stage_begin("prune_order", s);
   TG_TRY(locality_order(d, ord, &order, s));
   launch_row_norms(d, norms, s);
   stage_end("prune_order", s);
+  // candidate lists | two counters per batch; taken last and given back before the
+  // reverse edges, so that they ask for no memory the prune does not find
+  uint32_t batch = std::min(d.n, kSelectBatch), batches = 0;
+  for (;; batch /= 2) {
+    batches = (d.n + batch - 1) / batch;
+    const int rc = lists.alloc((size_t)batch * (lay.L() * 8 + 4) + (size_t)batches * 8);
+    if (rc == TAGORE_OK) break;
+    if (rc != TAGORE_ENOMEM || batch <= kMinBatch) return rc;
+  }
+  uint32_t* L_ids = lists.as<uint32_t>();
+  float* L_dis = reinterpret_cast<float*>(L_ids + (size_t)batch * lay.L());
+  uint32_t* L_cnt = reinterpret_cast<uint32_t*>(L_dis + (size_t)batch * lay.L());
+  uint32_t* ctr = L_cnt + batch;
+  TG_CUDA(cudaMemsetAsync(ctr, 0, (size_t)batches * 8, s));
   const char* sel_name = path ? "prune_select_path" : "prune_select_2hop";
   for (uint32_t i = 0; i < batches; ++i) {
     const uint32_t first = i * batch, cnt = std::min(batch, d.n - first);
@@ -1658,6 +1666,8 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
     stage_end("prune_filter", s);
     TG_CUDA(cudaGetLastError());
   }
+  rings.release();
+  lists.release();
   stage_begin("prune_reverse_store", s);
   TG_TRY(reverse_store(d, P_ids, reinterpret_cast<const uint32_t*>(P_dis), P_cnt, fd, 0, K, K, s));
   stage_end("prune_reverse_store", s);

@@ -1,0 +1,45 @@
+"""Calls on a device with little free memory: what a call can do without, it does
+without, with the same result."""
+import contextlib
+
+import numpy as np
+import pytest
+
+from tagore_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@contextlib.contextmanager
+def free_memory(capi, leave):
+    """Holds the device's free memory but `leave` bytes."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    capi.lib().tagore_trim_cache()
+    held = [torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")]
+    try:
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("mode,metric", [("path", "dist"), ("2-hop", "angle")])
+def test_prune_with_short_lists(capi, mode, metric):
+    # the candidate lists of 150,000 nodes take 692 MB at K = 96, the rest of the
+    # prune's scratch less than 200 MB
+    n, K, fd = 150_000, 96, 32
+    base, _ = synth.mixture("deep", n, 32, 75, 51)
+    st = capi.gnn_descent_host(base, K, 4)
+    ids, dis = st.download(0), st.download(3)
+    rows = []
+    for short in (False, True):
+        st.upload(0, ids)
+        st.upload(3, dis)
+        st.upload(5, np.zeros(n, np.uint32))
+        with free_memory(capi, 400 << 20) if short else contextlib.nullcontext():
+            capi.pruning_cfs(st, fd, mode, metric, topm=64, thre=0.5)
+        rows.append([st.download(i) for i in (0, 1, 3, 4, 5)])
+    st.free()
+    assert all(np.array_equal(a.view(np.uint32), b.view(np.uint32)) for a, b in zip(*rows))

@@ -737,35 +737,17 @@ static int join_exact(const knn::Work& w, uint32_t mode, cudaStream_t s) {
   return knn::join_plain(w, s);
 }
 
-int knn_build(const Dev& base, const float* norms, const KnnArgs& a, KnnStats* st, cudaStream_t s) {
+// The build of `d`, which is the caller's base or a padded copy of it; `dim` is the
+// base's width.
+static int build_rows(const Dev& d, uint32_t dim, const float* norms, const KnnArgs& a,
+                      KnnStats* st, cudaStream_t s) {
   using namespace knn;
-  Dev d = base;
-  if (d.n < 2 || a.k == 0 || a.k >= d.n) return fail(TAGORE_EINVAL, "need POINTS > K >= 1");
-  if (a.k > 128) return fail(TAGORE_EINVAL, "K must be <= 128 (got %u)", a.k);
-  if (d.dim % 4) return fail(TAGORE_EINVAL, "DIM must be a multiple of 4 (got %u)", d.dim);
-  if (d.n >= 0x7FFFFFFFu) return fail(TAGORE_EINVAL, "POINTS must be < 2^31");
-  if (a.mode > TAGORE_KNN_LEARNED) return fail(TAGORE_EINVAL, "unknown kNN mode %u", a.mode);
-  // The tensor-core joins gather rows with TMA, whose row stride is a multiple
-  // of 16 bytes. A width of 4 mod 8 is built on a copy of the base with one
-  // zero chunk per row: the same distances, and the exact join in place of the
-  // learned screen and the FP32 SIMT join it hands over to (50K x 100, K = 48,
-  // 10 iterations: 457 ms against 15.3 ms).
-  Scratch padded(s);
-  if (a.mode == TAGORE_KNN_CHOSEN && d.dim % 8 == 4 && d.dim < 1024) {
-    TG_TRY(padded.alloc((size_t)d.n * (d.dim + 4) * 2));
-    k_pad_rows<<<sm_count() * 8, 256, 0, s>>>(reinterpret_cast<const uint2*>(d.data), d.n,
-                                              d.dim / 4, padded.as<uint2>());
-    count_launch();
-    TG_CUDA(cudaGetLastError());
-    d.data = padded.as<__half>();
-    d.dim += 4;
-  }
   const uint32_t S = std::min<uint32_t>(a.sample ? a.sample : 32, kMaxS);
   // Partners kept per join row: 2, and 3 at the widths the learned screen used to
   // serve, whose builds had its proposals on top of the exact join's (50K x 100: mean
   // error of the distances 0.0066 with the screen, 0.0071 at T = 2, 0.0054 at T = 3).
-  const bool more = a.mode == TAGORE_KNN_CHOSEN && base.dim < 1024 &&
-                    (base.dim % 8 == 4 || (base.dim < 128 && base.dim % 16 != 0));
+  const bool more = a.mode == TAGORE_KNN_CHOSEN && dim < 1024 &&
+                    (dim % 8 == 4 || (dim < 128 && dim % 16 != 0));
   const uint32_t T = std::min<uint32_t>(a.per_row ? a.per_row : more ? 3 : 2,
                                         a.mode == TAGORE_KNN_PLAIN ? kMaxT : 4u);
   const uint32_t P = kPool;
@@ -930,6 +912,37 @@ int knn_build(const Dev& base, const float* norms, const KnnArgs& a, KnnStats* s
   sst.fallback = fallback ? 1u : 0u;
   set_screen_stats(sst);
   return TAGORE_OK;
+}
+
+int knn_build(const Dev& d, const float* norms, const KnnArgs& a, KnnStats* st, cudaStream_t s) {
+  using namespace knn;
+  if (d.n < 2 || a.k == 0 || a.k >= d.n) return fail(TAGORE_EINVAL, "need POINTS > K >= 1");
+  if (a.k > 128) return fail(TAGORE_EINVAL, "K must be <= 128 (got %u)", a.k);
+  if (d.dim % 4) return fail(TAGORE_EINVAL, "DIM must be a multiple of 4 (got %u)", d.dim);
+  if (d.n >= 0x7FFFFFFFu) return fail(TAGORE_EINVAL, "POINTS must be < 2^31");
+  if (a.mode > TAGORE_KNN_LEARNED) return fail(TAGORE_EINVAL, "unknown kNN mode %u", a.mode);
+  // The tensor-core joins gather rows with TMA, whose row stride is a multiple
+  // of 16 bytes. A width of 4 mod 8 is built on a copy of the base with one
+  // zero chunk per row: the same distances, and the exact join in place of the
+  // learned screen and the FP32 SIMT join it hands over to (50K x 100, K = 48,
+  // 10 iterations: 457 ms against 8.8 ms). A device without room for the copy
+  // keeps the screen, which needs none.
+  if (a.mode == TAGORE_KNN_CHOSEN && d.dim % 8 == 4 && d.dim < 1024) {
+    Scratch padded(s);
+    int rc = padded.alloc((size_t)d.n * (d.dim + 4) * 2);
+    if (rc == TAGORE_OK) {
+      Dev wide = d;
+      wide.data = padded.as<__half>();
+      wide.dim += 4;
+      k_pad_rows<<<sm_count() * 8, 256, 0, s>>>(reinterpret_cast<const uint2*>(d.data), d.n,
+                                                d.dim / 4, padded.as<uint2>());
+      count_launch();
+      TG_CUDA(cudaGetLastError());
+      rc = build_rows(wide, d.dim, norms, a, st, s);
+    }
+    if (rc != TAGORE_ENOMEM) return rc;
+  }
+  return build_rows(d, d.dim, norms, a, st, s);
 }
 
 }  // namespace tagore

@@ -743,12 +743,18 @@ static int build_rows(const Dev& d, uint32_t dim, const float* norms, const KnnA
                       KnnStats* st, cudaStream_t s) {
   using namespace knn;
   const uint32_t S = std::min<uint32_t>(a.sample ? a.sample : 32, kMaxS);
-  // Partners kept per join row: 2, and 3 at the widths the learned screen used to
-  // serve, whose builds had its proposals on top of the exact join's (50K x 100: mean
-  // error of the distances 0.0066 with the screen, 0.0071 at T = 2, 0.0054 at T = 3).
-  const bool more = a.mode == TAGORE_KNN_CHOSEN && dim < 1024 &&
-                    (dim % 8 == 4 || (dim < 128 && dim % 16 != 0));
-  const uint32_t T = std::min<uint32_t>(a.per_row ? a.per_row : more ? 3 : 2,
+  // Partners kept per join row: 2, and more at the widths the learned screen used to
+  // serve, whose builds had its proposals on top of the exact join's. Mean error of
+  // the distances with the screen, at T = 3 and at T = 4:
+  //   12,000 x 20, K = 32   0.0084  0.0095  0.0084
+  //   12,000 x 24, K = 32   0.0082  0.0087  0.0077
+  //   40,000 x 28, K = 48   0.0085  0.0090  0.0080
+  //   12,000 x 36, K = 32   0.0085  0.0073  0.0063
+  //   50,000 x 100, K = 48  0.0066  0.0054  (T = 2: 0.0071)
+  const bool screened = a.mode == TAGORE_KNN_CHOSEN && (dim % 8 == 4 || (dim < 128 && dim % 16 != 0));
+  const bool tc_width = tc_supported(d.dim) || tc_wide_supported(d.dim);
+  const uint32_t kept = !screened || !tc_width ? 2 : dim < 32 ? 4 : 3;
+  const uint32_t T = std::min<uint32_t>(a.per_row ? a.per_row : kept,
                                         a.mode == TAGORE_KNN_PLAIN ? kMaxT : 4u);
   const uint32_t P = kPool;
   const uint32_t K = a.k;
@@ -791,7 +797,6 @@ static int build_rows(const Dev& d, uint32_t dim, const float* norms, const KnnA
   count_launch();
   stage_end("knn_init", s, n64 * K * (2ull * d.dim + 8), n64 * K);
   TG_CUDA(cudaGetLastError());
-  const bool tc_width = tc_supported(d.dim) || tc_wide_supported(d.dim);
   const char* join_name = a.mode == TAGORE_KNN_PLAIN || !tc_width ? "knn_join_plain"
                           : tc_supported(d.dim)                   ? "knn_join_tc"
                                                                   : "knn_join_tc_wide";
@@ -927,7 +932,7 @@ int knn_build(const Dev& d, const float* norms, const KnnArgs& a, KnnStats* st, 
   // learned screen and the FP32 SIMT join it hands over to (50K x 100, K = 48,
   // 10 iterations: 457 ms against 8.8 ms). A device without room for the copy
   // keeps the screen, which needs none.
-  if (a.mode == TAGORE_KNN_CHOSEN && d.dim % 8 == 4 && d.dim < 1024) {
+  if (a.mode == TAGORE_KNN_CHOSEN && d.dim % 8 == 4 && d.dim > kTcMinDim && d.dim < 1024) {
     Scratch padded(s);
     int rc = padded.alloc((size_t)d.n * (d.dim + 4) * 2);
     if (rc == TAGORE_OK) {

@@ -1035,7 +1035,7 @@ int join_tc_wide(const Work& w, cudaStream_t s) {
 
 int join_tc(const Work& w, cudaStream_t s) {
   if (!tc_supported(w.dim))
-    return fail(TAGORE_EINVAL, "tensor-core join needs DIM in {8,16,..,128} (got %u)", w.dim);
+    return fail(TAGORE_EINVAL, "tensor-core join needs DIM in {16,24,..,128} (got %u)", w.dim);
   if (w.T > 4) return fail(TAGORE_EINVAL, "tensor-core join keeps at most 4 partners per row");
   CUtensorMap map;
   TG_TRY(make_row_map(&map, w.data, w.n, w.dim));

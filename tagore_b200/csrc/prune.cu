@@ -121,8 +121,18 @@ __device__ __noinline__ void beam_network(Beam bm, uint32_t off, uint32_t len, i
                });
 }
 
+// kSolo: the entry point's beam, one warp on an idle chip, which waits for latency
+// alone: its sorts are unrolled and its rows read by a lane each, all their loads at
+// once (at 1M x 128, K = 96, TOPM 64: 0.33 ms, with the collect's forms 0.45 ms).
+template <bool kSolo, int E>
+__device__ __forceinline__ void sort_keys(uint64_t (&key)[E], int lane) {
+  if constexpr (kSolo) knn::warp_sort_keys<E>(key, lane);
+  else knn::warp_sort_keys_rolled<E>(key, lane);
+}
+
 // Sorted (distance, position) keys of the n <= 128 entries at [off, off+n),
 // element-major in four registers per lane.
+template <bool kSolo>
 __device__ __forceinline__ void sorted_keys(const Beam& bm, uint32_t off, uint32_t n, uint64_t (&key)[4],
                                             int lane) {
 #pragma unroll
@@ -130,7 +140,7 @@ __device__ __forceinline__ void sorted_keys(const Beam& bm, uint32_t off, uint32
     const uint32_t j = lane + 32 * t;
     key[t] = j < n ? (((uint64_t)__float_as_uint(bm.dis[off + j]) << 32) | j) : ~0ull;
   }
-  knn::warp_sort_keys_rolled<4>(key, lane);
+  sort_keys<kSolo, 4>(key, lane);
 }
 
 __device__ __forceinline__ float key_dis(uint64_t k) { return __uint_as_float((uint32_t)(k >> 32)); }
@@ -138,7 +148,7 @@ __device__ __forceinline__ float key_dis(uint64_t k) { return __uint_as_float((u
 // Merges the m entering entries, whose (distance, slot) keys sit in sm/sid
 // [0, m), into the sorted prefix [0, topm) by rank, through the staging
 // arrays. Returns false (nothing moved) when two merged positions 0..topm tie.
-template <int E>
+template <bool kSolo, int E>
 __device__ __noinline__ bool beam_merge(Beam bm, uint32_t topm, uint32_t m, int lane) {
   uint64_t key[E];
 #pragma unroll
@@ -146,7 +156,7 @@ __device__ __noinline__ bool beam_merge(Beam bm, uint32_t topm, uint32_t m, int 
     const uint32_t q = lane + 32 * t;
     key[t] = q < m ? (((uint64_t)__float_as_uint(bm.sm[q]) << 32) | bm.sid[q]) : ~0ull;
   }
-  knn::warp_sort_keys_rolled<E>(key, lane);
+  sort_keys<kSolo, E>(key, lane);
 #pragma unroll
   for (int t = 0; t < E; ++t) {
     const uint32_t q = lane + 32 * t;
@@ -211,6 +221,7 @@ __device__ __noinline__ bool beam_merge(Beam bm, uint32_t topm, uint32_t m, int 
 // correct sort. With a full prefix only scored entries no farther than its
 // last one can reach positions 0..topm, so just those are sorted and merged
 // by rank; a tie there, or a prefix that is not full, runs the network.
+template <bool kSolo>
 __device__ __noinline__ void beam_update(Beam bm, uint32_t topm, uint32_t K, const uint32_t* fresh,
                             uint32_t nfresh, int lane) {
   const uint32_t W = topm + K;
@@ -243,14 +254,14 @@ __device__ __noinline__ void beam_update(Beam bm, uint32_t topm, uint32_t K, con
   if (m == 0) return;  // every scored entry lies beyond the prefix: nothing moves
   __syncwarp();
   bool ok;
-  if (m <= 32) ok = beam_merge<1>(bm, topm, m, lane);
-  else if (m <= 64) ok = beam_merge<2>(bm, topm, m, lane);
-  else ok = beam_merge<4>(bm, topm, m, lane);
+  if (m <= 32) ok = beam_merge<kSolo, 1>(bm, topm, m, lane);
+  else if (m <= 64) ok = beam_merge<kSolo, 2>(bm, topm, m, lane);
+  else ok = beam_merge<kSolo, 4>(bm, topm, m, lane);
   if (!ok) beam_network(bm, 0, W, lane);
 }
 
-// kWide: as warp_rows32's.
-template <bool kWide>
+// kSolo: as sort_keys'; kWide: as warp_rows32's, without a meaning for kSolo.
+template <bool kSolo, bool kWide>
 __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __restrict__ data,
                               uint32_t dim, uint32_t K, const __half* query, uint32_t start,
                               uint32_t topm, uint32_t iters, Beam bm, uint32_t* ring_id,
@@ -262,7 +273,7 @@ __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __re
     bm.ex[t] = 1;
   }
   __syncwarp();
-  const uint32_t own = rows32_of(lane);
+  const uint32_t own = kSolo ? lane : rows32_of(lane);
   uint32_t* fresh_at = reinterpret_cast<uint32_t*>(bm.sb);  // K <= 128 slots
   uint32_t curr = 0, to_explore = start;
   // Round 0 scores the start node's whole row (the seeds), the later ones the
@@ -310,7 +321,11 @@ __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __re
     __syncwarp();
     for (uint32_t base = 0; base < nfresh; base += 32) {
       const uint32_t r = base + own;
-      const float d = warp_rows32<kWide>(query, data, dim, bm.sid + base, min(32u, nfresh - base));
+      float d = 0.0f;
+      if constexpr (!kSolo)
+        d = warp_rows32<kWide>(query, data, dim, bm.sid + base, min(32u, nfresh - base));
+      else if (r < nfresh)
+        d = row_dist(query, data + (size_t)bm.sid[r] * dim, dim);
       if (r < nfresh) {
         bm.dis[topm + fresh_at[r]] = d;
         if (ring_id) {
@@ -324,7 +339,7 @@ __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __re
     curr += nfresh;
     __syncwarp();
     if (it > 0) {
-      beam_update(bm, topm, K, fresh_at, nfresh, lane);
+      beam_update<kSolo>(bm, topm, K, fresh_at, nfresh, lane);
       continue;
     }
     // Seeds: the network's order is observable on the first min(TOPM, K)
@@ -333,7 +348,7 @@ __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __re
     bool seeded = false;
     if (K <= 128) {
       uint64_t key[4];
-      sorted_keys(bm, topm, K, key, lane);
+      sorted_keys<kSolo>(bm, topm, K, key, lane);
       bool tie = false;
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
@@ -795,7 +810,6 @@ __global__ void k_validate(const uint32_t* __restrict__ g, size_t cnt, uint32_t 
 }
 
 // cal_ep_gpu (:1889-2058): one warp, 30 expansions from node 0 toward the centre.
-template <bool kWide>
 __global__ void k_cal_ep(const uint32_t* __restrict__ G, const __half* __restrict__ data,
                          const __half* __restrict__ center, uint32_t dim, uint32_t K,
                          uint32_t topm, uint32_t* ep) {
@@ -803,8 +817,8 @@ __global__ void k_cal_ep(const uint32_t* __restrict__ G, const __half* __restric
   Beam bm = beam_carve(smem, topm, K);
   const int lane = threadIdx.x & 31;
   if (threadIdx.x >= 32) return;
-  const uint32_t best = warp_beam<kWide>(G, data, dim, K, center, 0, topm, 30, bm, nullptr, nullptr,
-                                         nullptr, lane);
+  const uint32_t best = warp_beam<true, true>(G, data, dim, K, center, 0, topm, 30, bm, nullptr,
+                                              nullptr, nullptr, lane);
   if (lane == 0) *ep = best;
 }
 
@@ -833,7 +847,7 @@ __device__ __forceinline__ uint32_t collect_node(
   uint32_t scored = kSelectCand;  // 2-hop: the 480 collected
   if (kPath) {
     uint32_t curr = 0;
-    warp_beam<kWide>(G, data, dim, K, q, ep, topm, 10, bm, rid, rds, &curr, lane);
+    warp_beam<false, kWide>(G, data, dim, K, q, ep, topm, 10, bm, rid, rds, &curr, lane);
     scored = curr;
     __syncwarp();  // the ring (global) and the beam's region are done
     for (uint32_t i = lane; i < kSelectCand; i += 32) {
@@ -1564,10 +1578,9 @@ constexpr uint32_t kSelectBatch = 1u << 18, kMinBatch = 1u << 9;
 bool on_16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 int launch_cal_ep(const Dev& d, uint32_t topm, uint32_t* ep_dev, cudaStream_t s) {
-  auto* fn = on_16(d.data) && on_16(d.center) ? k_cal_ep<true> : k_cal_ep<false>;
   const size_t sm = beam_bytes(topm, d.k);
-  TG_TRY(set_smem((const void*)fn, sm));
-  fn<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, d.k, topm, ep_dev);
+  TG_TRY(set_smem((const void*)k_cal_ep, sm));
+  k_cal_ep<<<1, 32, sm, s>>>(d.graph, d.data, d.center, d.dim, d.k, topm, ep_dev);
   count_launch();
   TG_CUDA(cudaGetLastError());
   return TAGORE_OK;

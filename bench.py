@@ -313,8 +313,8 @@ def main():
             r["dram_gbs"] = traffic / (ms_l * 1e-3) / 1e9
             r["dram_frac"] = r["dram_gbs"] / peak
         if name == "knn_join_tc":
-            # every node join is one full 128 x 128 x d FP16 Gram tile on tcgen05
-            flops = 2.0 * 128 * 128 * dim * n
+            # the joins' 128 x 128 x d FP16 Gram tiles on tcgen05, as the kernels count them
+            flops = 2.0 * 128 * 128 * dim * stages["knn_join_tiles"][3] / max(1, s_launch)
             r["tensor_tflops"] = flops / (ms_l * 1e-3) / 1e12
             r["tensor_peak_tflops"] = tflops_peak
             r["tensor_frac"] = r["tensor_tflops"] / tflops_peak
@@ -428,7 +428,7 @@ def main():
                 "chosen_speedup_vs_plain": (plain_ms / ms) if plain_ms else None,
                 "roofline": roofline(name),
                 "roofline_next": [roofline(k) for k in ranked[1:3]],
-                "stages_ms_per_step": {k: v[0] / a.steps for k, v in stages.items()},
+                "stages_ms_per_step": {k: v[0] / a.steps for k, v in stages.items() if v[1]},
                 "gpu_launches": launches,
                 "clocks": clocks, "e2e": e2e, "cpu_baseline": cpu}
         line.update(extra)

@@ -900,7 +900,7 @@ static int build_rows(const Dev& d, uint32_t dim, const float* norms, const KnnA
   k_finalize<<<sms * 8, 256, 0, s>>>(w.nb, d.n, K, d.graph, d.nd);
   count_launch();
   TG_CUDA(cudaGetLastError());
-  unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  unsigned long long h[11] = {};
   TG_CUDA(cudaMemcpyAsync(h, w.stats, sizeof(h), cudaMemcpyDeviceToHost, s));
   TG_CUDA(cudaStreamSynchronize(s));
   if ((uint32_t)h[4] != 0) return fail(TAGORE_ETIMEOUT, "tensor-core join: a bounded wait ran out");
@@ -908,6 +908,7 @@ static int build_rows(const Dev& d, uint32_t dim, const float* norms, const KnnA
   // distance record, list id), one 8-byte count pair per node, one 8-byte
   // read-modify-write per proposal
   stage_add(join_name, h[3] * (2ull * d.dim + 12) + n64 * a.iters * 8 + h[0] * 16, h[1]);
+  if (h[10]) stage_add("knn_join_tiles", 0, h[10]);  // 128-row tiles of all iterations
   if (st) {
     st->proposals = h[0];
     st->pairs = h[1];

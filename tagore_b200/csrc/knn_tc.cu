@@ -391,7 +391,7 @@ __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* 
                               const uint32_t* __restrict__ lists,
                               const uint32_t* __restrict__ lcnt, uint32_t n, uint32_t dim,
                               uint32_t K, unsigned long long* n_rows,
-                              const uint32_t* __restrict__ order) {
+                              unsigned long long* n_tiles, const uint32_t* __restrict__ order) {
   const uint32_t lane = threadIdx.x & 31u, blocks = (dim + 63) / 64;
   NodeWindow win{blockIdx.x};
   uint32_t ph_empty[kStages] = {};
@@ -425,6 +425,7 @@ __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* 
                    "r"(group_bytes(p) * blocks)
                    : "memory");
       *n_rows += p.tot[0] + p.tot[1];
+      ++*n_tiles;
       s.filled = j + 1;
     }
     __syncwarp();
@@ -487,10 +488,10 @@ __global__ void __launch_bounds__(kThreads, 3)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = s.taddr;
-  unsigned long long n_pairs = 0, n_props = 0, n_rows = 0;
+  unsigned long long n_pairs = 0, n_props = 0, n_rows = 0, n_tiles = 0;
 
   if (warp == kConsumers / 32) {
-    join_producer<D>(s, tmap, meta, lists, lcnt, n, dim, K, &n_rows, order);
+    join_producer<D>(s, tmap, meta, lists, lcnt, n, dim, K, &n_rows, &n_tiles, order);
   } else {
     uint32_t ph_full[kStages] = {}, ph_mma[2] = {0, 0};
     bool pending[2] = {false, false};  // thread 0: committed MMAs not yet waited for
@@ -603,6 +604,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   if (n_props) atomicAdd(&stats[0], n_props);
   if (n_pairs) atomicAdd(&stats[1], n_pairs);
   if (n_rows) atomicAdd(&stats[3], n_rows);
+  if (n_tiles) atomicAdd(&stats[10], n_tiles);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)
@@ -650,7 +652,7 @@ __device__ void wide_producer(WideSmem& s, const CUtensorMap& tmap, const float2
                               const uint32_t* __restrict__ lists,
                               const uint32_t* __restrict__ lcnt, uint32_t n, uint32_t dim,
                               uint32_t K, unsigned long long* n_rows,
-                              const uint32_t* __restrict__ order) {
+                              unsigned long long* n_tiles, const uint32_t* __restrict__ order) {
   const uint32_t lane = threadIdx.x & 31u, blocks = (dim + 63) / 64;
   NodeWindow win{blockIdx.x};
   uint32_t fill = 0;
@@ -678,6 +680,7 @@ __device__ void wide_producer(WideSmem& s, const CUtensorMap& tmap, const float2
     if (lane == 0) {
       set_slot(s.slot[ns], p);
       *n_rows += p.tot[0] + p.tot[1];
+      ++*n_tiles;
     }
     load_rows(p, meta, lists, lane, s.ids[ns], s.hnrm[ns], s.kth[ns]);
     __syncwarp();
@@ -810,10 +813,10 @@ __global__ void __launch_bounds__(kWideThreads, 2)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = s.taddr;
-  unsigned long long n_pairs = 0, n_props = 0, n_rows = 0;
+  unsigned long long n_pairs = 0, n_props = 0, n_rows = 0, n_tiles = 0;
 
   if (warp == 4) {
-    wide_producer(s, tmap, meta, lists, lcnt, n, dim, K, &n_rows, order);
+    wide_producer(s, tmap, meta, lists, lcnt, n, dim, K, &n_rows, &n_tiles, order);
   } else if (warp == 5) {
     if ((tid & 31u) == 0) wide_mma(s, tmem, dim);
     __syncwarp();
@@ -923,6 +926,7 @@ __global__ void __launch_bounds__(kWideThreads, 2)
   if (n_props) atomicAdd(&stats[0], n_props);
   if (n_pairs) atomicAdd(&stats[1], n_pairs);
   if (n_rows) atomicAdd(&stats[3], n_rows);
+  if (n_tiles) atomicAdd(&stats[10], n_tiles);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)

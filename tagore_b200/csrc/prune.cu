@@ -658,7 +658,7 @@ static __device__ __noinline__ bool exact_test(const __half* __restrict__ data, 
 
 // Filter stage over a compacted list (warp_compact) by one warp. Returns the
 // number of ids the reference stores: one less than its selection steps (:1462,
-// :1623).
+// :1623). *tested: the candidates taken before the degree was full.
 //
 // The list is taken 32 candidates at a time. A tile is first tested against the
 // kept neighbours (16 per screen, stopping when no candidate is left), then its
@@ -673,11 +673,12 @@ __device__ __forceinline__ uint32_t warp_filter(const uint32_t* cand, const floa
                                                 uint32_t len, bool tail, uint32_t fd, int metric,
                                                 float thre, const __half* __restrict__ data,
                                                 const float* __restrict__ norms, uint32_t dim,
-                                                const Kept& k, int lane) {
+                                                const Kept& k, int lane,
+                                                uint32_t* tested = nullptr) {
   const ScreenRule rule{metric, thre, screen_eps(dim)};
   const unsigned below = (1u << lane) - 1u;
-  uint32_t nsel = 0, last = 0;
-  for (uint32_t base = 0; base < len && nsel < fd; base += 32) {
+  uint32_t nsel = 0, last = 0, base = 0;
+  for (; base < len && nsel < fd; base += 32) {
     const uint32_t i = base + lane;
     uint32_t c = kInv;
     float dc = 0.0f, nc = 0.0f;
@@ -755,6 +756,7 @@ __device__ __forceinline__ uint32_t warp_filter(const uint32_t* cand, const floa
     __syncwarp();
   }
   __syncwarp();
+  if (tested) *tested = min(base, len);
   if (nsel == fd) return fd - 1;
   if (nsel >= 2 && last == len - 1 && tail) return nsel - 1;
   return nsel;
@@ -888,8 +890,9 @@ __device__ __forceinline__ uint32_t collect_node(
 
 // The filter half: select_path and select_2hop always use distance_filter and
 // angle_filter respectively. Results go to scratch rows, and the selected
-// distances to the node's own nd row, which no other node reads.
-__device__ __forceinline__ void filter_node(const uint32_t* cand, const float* cdis, uint32_t len,
+// distances to the node's own nd row, which no other node reads. Returns the
+// candidates tested.
+__device__ __forceinline__ uint32_t filter_node(const uint32_t* cand, const float* cdis, uint32_t len,
                                             bool tail, uint32_t fd, int metric, float thre,
                                             const __half* __restrict__ data,
                                             const float* __restrict__ norms, uint32_t dim,
@@ -897,8 +900,9 @@ __device__ __forceinline__ void filter_node(const uint32_t* cand, const float* c
                                             float* __restrict__ nd, uint32_t* __restrict__ P_ids,
                                             float* __restrict__ P_dis,
                                             uint32_t* __restrict__ P_cnt, int lane) {
+  uint32_t tested = 0;
   const uint32_t stored =
-      warp_filter(cand, cdis, len, tail, fd, metric, thre, data, norms, dim, k, lane);
+      warp_filter(cand, cdis, len, tail, fd, metric, thre, data, norms, dim, k, lane, &tested);
   for (uint32_t i = lane; i < stored; i += 32) {
     P_ids[(size_t)b * fd + i] = k.id[i];
     P_dis[(size_t)b * fd + i] = k.dis[i];
@@ -906,6 +910,7 @@ __device__ __forceinline__ void filter_node(const uint32_t* cand, const float* c
   }
   if (lane == 0) P_cnt[b] = stored;
   __syncwarp();
+  return tested;
 }
 
 // The list as it was collected, sorted by the network: where warp_list cannot decide.
@@ -981,7 +986,7 @@ __global__ void __launch_bounds__(kWarps * 32, 7)
     uint32_t got = warp_list(cand, cdis, mark, K, b, out_ids, out_dis, lane);
     if (got == kInv)
       got = network_list<kPath>(G, K, scored, rid, rds, cand, cdis, b, out_ids, out_dis, lane);
-    rows += scored + (got & ~kTailBit);
+    rows += scored;
     if (lane == 0) L_cnt[i] = got;
     __syncwarp();
   }
@@ -994,14 +999,22 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
              const __half* __restrict__ data, const float* __restrict__ norms, uint32_t first,
              uint32_t cnt, uint32_t dim, uint32_t K, uint32_t* __restrict__ ctr, uint32_t fd,
              int metric, float thre, uint32_t* __restrict__ P_ids, float* __restrict__ P_dis,
-             uint32_t* __restrict__ P_cnt, const uint32_t* __restrict__ order) {
+             uint32_t* __restrict__ P_cnt, unsigned long long* __restrict__ work,
+             const uint32_t* __restrict__ order) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Kept k = kept_carve(smem + (size_t)warp * kept_bytes(fd), fd);
+  uint32_t listed = 0, tested = 0;  // below 2^28 each, a batch's lists
   for (uint32_t i = next_node(ctr, lane); i < cnt; i = next_node(ctr, lane)) {
     const uint32_t b = node_at(order, first + i), lc = L_cnt[i];
-    filter_node(L_ids + (size_t)i * L, L_dis + (size_t)i * L, lc & ~kTailBit, (lc & kTailBit) != 0,
-                fd, metric, thre, data, norms, dim, k, b, K, nd, P_ids, P_dis, P_cnt, lane);
+    listed += lc & ~kTailBit;
+    tested += filter_node(L_ids + (size_t)i * L, L_dis + (size_t)i * L, lc & ~kTailBit,
+                          (lc & kTailBit) != 0, fd, metric, thre, data, norms, dim, k, b, K, nd,
+                          P_ids, P_dis, P_cnt, lane);
+  }
+  if (lane == 0) {
+    atomicAdd(work, (unsigned long long)listed);
+    atomicAdd(work + 1, (unsigned long long)tested);
   }
 }
 
@@ -1612,11 +1625,12 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   if (path && (a.topm == 0 || a.topm > 256)) return fail(TAGORE_EINVAL, "TOPM must be in [1, 256]");
   const SelLayout lay{path ? a.topm : 0u, K, 0};
   Scratch sc(s);
-  // [u64 rows scored][u32 entry point][u32 unused] | select rows | norms
-  const size_t head = 16;
+  // [u64 rows scored, candidates listed, candidates tested][u32 entry point][u32 unused]
+  // | select rows | norms
+  const size_t head = 32;
   TG_TRY(sc.alloc(head + (size_t)d.n * fd * 8 + (size_t)d.n * 8));
   unsigned long long* work = sc.as<unsigned long long>();
-  uint32_t* ep_dev = reinterpret_cast<uint32_t*>(work + 1);
+  uint32_t* ep_dev = reinterpret_cast<uint32_t*>(work + 3);
   uint32_t* P_ids = reinterpret_cast<uint32_t*>(sc.as<unsigned char>() + head);
   float* P_dis = reinterpret_cast<float*>(P_ids + (size_t)d.n * fd);
   uint32_t* P_cnt = reinterpret_cast<uint32_t*>(P_dis + (size_t)d.n * fd);
@@ -1674,7 +1688,7 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
     stage_begin("prune_filter", s);
     k_filter<<<gridf, kWarps * 32, smf, s>>>(L_ids, L_dis, L_cnt, lay.L(), d.nd, d.data, norms, first,
                                              cnt, d.dim, K, ctr + 2 * i + 1, fd, path ? 0 : 1,
-                                             a.thre, P_ids, P_dis, P_cnt, order);
+                                             a.thre, P_ids, P_dis, P_cnt, work + 1, order);
     count_launch();
     stage_end("prune_filter", s);
     TG_CUDA(cudaGetLastError());
@@ -1692,14 +1706,17 @@ int run_dist_prune(const Dev& d, const PruneArgs& a, bool path, int metric, uint
   if (path && ep_host) {
     TG_CUDA(cudaMemcpyAsync(ep_host, ep_dev, 4, cudaMemcpyDeviceToHost, s));
   }
-  unsigned long long rows = 0;
-  if (profiling()) TG_CUDA(cudaMemcpyAsync(&rows, work, 8, cudaMemcpyDeviceToHost, s));
+  unsigned long long w[3] = {0, 0, 0};
+  if (profiling()) TG_CUDA(cudaMemcpyAsync(w, work, sizeof(w), cudaMemcpyDeviceToHost, s));
   TG_CUDA(cudaStreamSynchronize(s));
-  // select traffic: every scored row and every listed candidate's row (2d
-  // bytes), the kNN row and distances read (8 B per slot), the selected ids and
-  // distances written (8 B each)
-  if (profiling())
-    stage_add(sel_name, rows * 2ull * d.dim + (uint64_t)d.n * (8ull * K + 8ull * fd + 4), d.n);
+  if (profiling()) {
+    // collect: every scored row (2d bytes), the kNN row and its distances in, the
+    // list out; filter: the tested candidates' entries and rows in, the selected ids
+    // and distances out (8 bytes an entry throughout)
+    const uint64_t row = 2ull * d.dim, n = d.n;
+    stage_add(sel_name, w[0] * row + n * 8 * K + w[1] * 8, n);
+    stage_add("prune_filter", w[2] * (row + 8) + n * (8ull * fd + 4), n);
+  }
   return TAGORE_OK;
 }
 

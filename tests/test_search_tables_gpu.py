@@ -47,3 +47,19 @@ def test_widths(capi, orc, dim):
     offs, adj = ragged_graph(n, 40, np.random.default_rng(dim))
     got, want = both(capi, orc, base_of(n, dim, 5), offs, adj, 5, base_of(33, dim, 6), 50, 20, 9)
     assert np.array_equal(got, want)
+
+
+# ids of 25 bits take a shared table of 2,048 buckets so that a remainder fits 14 bits;
+# ids of 26 bits leave the shared table out, and every visited id is in global memory
+@pytest.mark.parametrize("n", [(1 << 24) + 1, (1 << 25) + 1])
+@pytest.mark.parametrize("seed", [0, 5])
+def test_bases_at_the_shared_tables_limit(capi, orc, n, seed):
+    rng = np.random.default_rng(n)
+    base = rng.integers(0, 50, (n, 4), dtype=np.uint8).astype(np.float32)
+    offs = np.arange(0, 3 * n + 1, 3, dtype=np.uint64)
+    adj = rng.integers(0, n, 3 * n, dtype=np.uint32)
+    adj[::5] = n - 1 - adj[::5] % 1000  # the highest ids, met again and again
+    q = rng.integers(0, 50, (24, 4)).astype(np.float32)
+    for L in (50, 1500):
+        got, want = both(capi, orc, base, offs, adj, n - 1, q, L, 20, seed)
+        assert np.array_equal(got, want)

@@ -348,6 +348,12 @@ static __device__ __noinline__ float row_dist(const __half* __restrict__ a,
 // loads at 96 dims took 1.8 times the instructions.
 // Collect with these, chained membership and rolled sorts: 1M x 128, K = 96, 98.4 ->
 // 79.6 ms; 500K x 96, K = 64, 32.1 -> 29.4 ms.
+//
+// warp_rows32_fixed holds a lane's units in registers, at the two widths up to 128
+// that the configurations have: the collect takes 18.4 ms with it and 25.4 ms without
+// at 300K x 128, 29.0 and 39.2 ms at 500K x 96. Each width is one more copy in code
+// that waits for instructions (5.2 of 13.8 stall cycles per issue), so the others
+// share warp_rows32_any (300K x 64: 21.4 ms, 300K x 112: 25.5 ms).
 __device__ __forceinline__ uint32_t rows32_of(int lane) {
   return 8 * ((uint32_t)lane & 3u) + ((uint32_t)lane >> 2);
 }

@@ -59,7 +59,7 @@ struct __align__(1024) TcSmem {
   uint32_t warp_pairs[kConsumers / 32];
   unsigned long long full_bar[kStages];   // rows landed and stage filled
   unsigned long long empty_bar[kStages];  // consumers done with the stage
-  unsigned long long mma_bar[2];          // accumulator written
+  unsigned long long mma_bar;             // accumulator written
   uint32_t taddr;
   NodeSlot slot[kStages];
   uint32_t filled, consumed;  // producer fills with rows; fills the consumers saw land
@@ -166,7 +166,11 @@ __device__ __forceinline__ float key_max(float a, float b) {
 // column number sits in the value's seven lowest bits (2^-16 of the distance, far
 // inside the 2^-12 margin; the kept pairs are ranked exactly afterwards), so the
 // best T are kept by min and max alone, with no branch: with an insertion branch
-// most columns of an early iteration had some lane that took it.
+// most columns of an early iteration had some lane that took it. Which of two columns
+// within 2^-16 of one another is kept may differ from the full value's choice; the
+// distances' mean error over six builds each does not (40K points, K = 48: 16 dims
+// 0.01488 before and after, 32: 0.01044 and 0.01045, 64: 0.00868, 128: 0.00714, 256:
+// 0.00565).
 // 1M x 128, K = 64, 10 iterations: the build 205 -> 178 ms; 165K x 96, 16 iterations:
 // 40.7 -> 33.6 ms; 250K x 960: 184.9 -> 178.2 ms.
 template <int T>
@@ -386,11 +390,10 @@ __device__ __forceinline__ bool group_rows(const NodePair& p, const uint32_t* id
 // ids, norms and k-th distances (one packed record per row) by the lanes, rows by
 // TMA tile::gather4. Runs kStages tiles ahead of the consumers; ends by publishing
 // a slot that is not live.
-template <int D>
 __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* __restrict__ meta,
                               const uint32_t* __restrict__ lists,
                               const uint32_t* __restrict__ lcnt, uint32_t n, uint32_t dim,
-                              uint32_t K, unsigned long long* n_rows,
+                              unsigned long long* n_rows,
                               unsigned long long* n_tiles, const uint32_t* __restrict__ order) {
   const uint32_t lane = threadIdx.x & 31u, blocks = (dim + 63) / 64;
   NodeWindow win{blockIdx.x};
@@ -451,13 +454,14 @@ __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* 
 // i - 1; every thread owns one tile row, screens it from TMEM and re-ranks the
 // kept pairs exactly. Three blocks per SM (12 consumer warps) with one
 // 128-column accumulator each hide more latency than two blocks with two
-// accumulators each (240 against 312 ms for the 1M x 128 build's ten joins).
+// accumulators each: 240 against 312 ms for ten joins at 1M x 128, K = 96, when that
+// was chosen; they take 105 ms now.
 template <int D>
 __global__ void __launch_bounds__(kThreads, 3)
     k_join_tc(const __grid_constant__ CUtensorMap tmap, const float2* __restrict__ meta,
               const uint32_t* __restrict__ lists,
-              const uint32_t* __restrict__ lcnt, uint32_t n, uint32_t dim, uint32_t K, uint32_t T,
-              uint32_t P, unsigned long long* __restrict__ pool,
+              const uint32_t* __restrict__ lcnt, uint32_t n, uint32_t dim, uint32_t T, uint32_t P,
+              unsigned long long* __restrict__ pool,
               unsigned long long* __restrict__ stats, int* __restrict__ err,
               const uint32_t* __restrict__ order) {
   extern __shared__ unsigned char smem_raw[];
@@ -476,8 +480,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s.full_bar[st])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&s.empty_bar[st])));
     }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s.mma_bar[0])));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s.mma_bar[1])));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s.mma_bar)));
     asm volatile("fence.mbarrier_init.release.cluster;");
     asm volatile("fence.proxy.async.shared::cta;");
     s.flag = 1;
@@ -491,13 +494,13 @@ __global__ void __launch_bounds__(kThreads, 3)
   unsigned long long n_pairs = 0, n_props = 0, n_rows = 0, n_tiles = 0;
 
   if (warp == kConsumers / 32) {
-    join_producer<D>(s, tmap, meta, lists, lcnt, n, dim, K, &n_rows, &n_tiles, order);
+    join_producer(s, tmap, meta, lists, lcnt, n, dim, &n_rows, &n_tiles, order);
   } else {
-    uint32_t ph_full[kStages] = {}, ph_mma[2] = {0, 0};
-    bool pending[2] = {false, false};  // thread 0: committed MMAs not yet waited for
+    uint32_t ph_full[kStages] = {}, ph_mma = 0;
+    bool pending = false;  // thread 0: committed MMAs not yet waited for
     // Thread 0: waits for stage st's rows (phase ph) and issues their Gram
-    // tile into accumulator acc. No MMA for a stage that is not live or on timeout.
-    auto issue = [&](int st, uint32_t ph, uint32_t acc) {
+    // tile into the accumulator. No MMA for a stage that is not live or on timeout.
+    auto issue = [&](int st, uint32_t ph) {
       if (!mbar_wait_bounded(smem_u32(&s.full_bar[st]), ph)) {
         s.flag = 0;
         return;
@@ -510,28 +513,27 @@ __global__ void __launch_bounds__(kThreads, 3)
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + acc * 128),
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
             "l"(desc), "l"(desc), "r"(kIdesc), "r"(accum));
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(&s.mma_bar[acc])));
-      pending[acc] = true;
+          smem_u32(&s.mma_bar)));
+      pending = true;
     };
-    if (tid == 0) issue(0, 0, 0);
+    if (tid == 0) issue(0, 0);
     const uint32_t r = tid, lane = tid & 31u;
     uint32_t got_full = 0;  // nodes whose rows this thread has seen land
     for (uint32_t i = 0;; ++i) {
       const int st = (int)(i % kStages);
-      const uint32_t acc = 0u;  // one accumulator, refilled once the screen has read it
       const bool got = mbar_wait_bounded(smem_u32(&s.full_bar[st]), ph_full[st]);
       ph_full[st] ^= 1u;
       got_full += got ? 1u : 0u;
       const bool done = got && !s.slot[st].live;
       bool ok = got;
       if (got && !done) {
-        ok = mbar_wait_bounded(smem_u32(&s.mma_bar[acc]), ph_mma[acc]);
-        ph_mma[acc] ^= 1u;
-        pending[acc] = false;
+        ok = mbar_wait_bounded(smem_u32(&s.mma_bar), ph_mma);
+        ph_mma ^= 1u;
+        pending = false;
       }
       // every consumer leaves together: on any thread's timeout, or at the end
       if (consumers_any(!ok)) {
@@ -542,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       asm volatile("tcgen05.fence::after_thread_sync;");
       // ---- screen: each thread owns one row ----
       uint32_t bc[4];
-      screen_rows(T, tmem + acc * 128, s.hnrm[st], s.hnrm[st][r], s.kth[st][r], r, s.slot[st], bc);
+      screen_rows(T, tmem, s.hnrm[st], s.hnrm[st][r], s.kth[st][r], r, s.slot[st], bc);
       // kept pairs go to one list so that the exact re-rank is shared evenly
       uint32_t kept = 0;
 #pragma unroll
@@ -559,7 +561,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       consumers_sync();
       if (tid == 0) {
         const int st1 = (int)((i + 1) % kStages);
-        issue(st1, ph_full[st1], 0u);  // the phase node i + 1 completes
+        issue(st1, ph_full[st1]);  // the phase node i + 1 completes
       }
       uint32_t off = incl - kept, npairs = 0;
 #pragma unroll
@@ -587,8 +589,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
     if (tid == 0) {
       // MMAs committed but not consumed (only after a timeout) land first
-      for (int a = 0; a < 2; ++a)
-        if (pending[a]) mbar_wait_bounded(smem_u32(&s.mma_bar[a]), ph_mma[a]);
+      if (pending) mbar_wait_bounded(smem_u32(&s.mma_bar), ph_mma);
       s.consumed = got_full;
     }
   }
@@ -651,7 +652,7 @@ struct __align__(1024) WideSmem {
 __device__ void wide_producer(WideSmem& s, const CUtensorMap& tmap, const float2* __restrict__ meta,
                               const uint32_t* __restrict__ lists,
                               const uint32_t* __restrict__ lcnt, uint32_t n, uint32_t dim,
-                              uint32_t K, unsigned long long* n_rows,
+                              unsigned long long* n_rows,
                               unsigned long long* n_tiles, const uint32_t* __restrict__ order) {
   const uint32_t lane = threadIdx.x & 31u, blocks = (dim + 63) / 64;
   NodeWindow win{blockIdx.x};
@@ -777,7 +778,7 @@ __device__ void wide_mma(WideSmem& s, uint32_t tmem, uint32_t dim) {
 __global__ void __launch_bounds__(kWideThreads, 2)
     k_join_tc_wide(const __grid_constant__ CUtensorMap tmap, const __half* __restrict__ data,
                    const float2* __restrict__ meta, const uint32_t* __restrict__ lists, const uint32_t* __restrict__ lcnt,
-                   uint32_t n, uint32_t dim, uint32_t K, uint32_t T, uint32_t P,
+                   uint32_t n, uint32_t dim, uint32_t T, uint32_t P,
                    unsigned long long* __restrict__ pool, unsigned long long* __restrict__ stats,
                    int* __restrict__ err, const uint32_t* __restrict__ order) {
   extern __shared__ unsigned char smem_raw[];
@@ -816,7 +817,7 @@ __global__ void __launch_bounds__(kWideThreads, 2)
   unsigned long long n_pairs = 0, n_props = 0, n_rows = 0, n_tiles = 0;
 
   if (warp == 4) {
-    wide_producer(s, tmap, meta, lists, lcnt, n, dim, K, &n_rows, &n_tiles, order);
+    wide_producer(s, tmap, meta, lists, lcnt, n, dim, &n_rows, &n_tiles, order);
   } else if (warp == 5) {
     if ((tid & 31u) == 0) wide_mma(s, tmem, dim);
     __syncwarp();
@@ -994,7 +995,7 @@ int launch(const Work& w, const CUtensorMap& map, cudaStream_t s) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int* err = reinterpret_cast<int*>(w.stats + 4);
   k_join_tc<D><<<sms * 3, kThreads, sm, s>>>(map, w.meta, w.lists, w.lcnt, w.n, w.dim,
-                                             w.K, w.T, w.P, w.pool, w.stats, err, w.order);
+                                             w.T, w.P, w.pool, w.stats, err, w.order);
   TG_CUDA(cudaGetLastError());
   return TAGORE_OK;
 }
@@ -1008,7 +1009,7 @@ int launch_wide(const Work& w, const CUtensorMap& map, cudaStream_t s) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int* err = reinterpret_cast<int*>(w.stats + 4);
   k_join_tc_wide<<<sms * 2, kWideThreads, sm, s>>>(map, w.data, w.meta, w.lists, w.lcnt,
-                                                    w.n, w.dim, w.K, w.T, w.P, w.pool, w.stats, err,
+                                                    w.n, w.dim, w.T, w.P, w.pool, w.stats, err,
                                                     w.order);
   TG_CUDA(cudaGetLastError());
   return TAGORE_OK;

@@ -35,7 +35,6 @@ constexpr int kWarps = 4;  // warps (= nodes in flight) per block
 
 
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // Beam search shared by cal_ep_gpu (:1905-2047) and collect_path (:1211-1335).
 // The helpers below are __noinline__ and their sorts rolled: the warps sit in
 // different phases, so one small copy of each sort and merge keeps the code they
@@ -946,8 +945,8 @@ static __device__ __noinline__ uint32_t network_list(const uint32_t* __restrict_
 // ring_ids / ring_dis: per-warp rings of kSelectCand scored nodes (path), by the
 // warp's global number.
 //
-// Collect and filter are two kernels with the list between them in memory
-// (about 4 KB written and read per node, 1.4 ms of a 1M prune): the beam waits on
+// Collect and filter are two kernels with the list between them in memory (about
+// 4.6 KB of it per node at K = 96, 1.4 ms of a 1M prune): the beam waits on
 // gathers and wants warps, the filter's tiles want registers, and each half's
 // code fits the instruction cache.
 template <bool kPath, bool kWide>
@@ -1247,9 +1246,9 @@ __global__ void __launch_bounds__(kWarps * 32)
 
 // collect_1hop + filter_dpg (:1713-1785): detour[m] counts earlier a with
 // d(n_a, n_m) < d(u, n_m), over the reference's pair set (all a < m but the
-// middle row of an odd K, :1715-1717), each warp using its own vector (see
-// header note). The pairs are screened 32 positions against 16 earlier ones at a
-// time; the few ambiguous ones take the exact distance.
+// middle row of an odd K, :1715-1717), each warp with vectors of its own (the
+// reference's warps race on one in shared memory). The pairs are screened 32 positions
+// against 16 earlier ones at a time; the few ambiguous ones take the exact distance.
 //
 // Bound by the row gathers, mostly from L1.
 __host__ __device__ inline uint32_t dpg_words(uint32_t K) { return 4 * K + kScreenFloats; }

@@ -25,7 +25,7 @@ namespace tagore {
 // the group norms' product; over the groups that is 64 * 2^-23 * (n_r + n_q) / 2,
 // so 2 g is within 2^-17 (n_r + n_q). The FP32 sum of the groups adds
 // (d / 64) 2^-24, the two norms 2^-18.7 and the reference-order distance itself
-// (at most 2 (n_r + n_q)) 2^-18.5: in all 1.3e-5, below 2^-16 = 1.53e-5.
+// (at most 2 (n_r + n_q)) 2^-18.5: in all 1.37e-5, below 2^-16 = 1.53e-5.
 constexpr float kScreenEps = 1.52587890625e-05f;
 
 __host__ __device__ inline float screen_eps(uint32_t dim) {

@@ -68,9 +68,11 @@ def tensor_peak():
 # What limits each kernel, from its ncu captures (profiles/): the roofline
 # class stays the HBM roofline of a gather kernel, this names the binding.
 BINDING = {
-    "prune_select_path": "latency: dependent L2-hit row gathers per warp step (long_scoreboard); "
-                         "DRAM traffic well below the HBM roofline",
-    "knn_join_tc": "latency and barriers: per-node TMA gathers from L2 and the consumer "
+    "prune_select_path": "instruction fetch (no_instruction), then dependent L2-hit row gathers "
+                         "(long_scoreboard); DRAM traffic well below the HBM roofline",
+    "prune_filter": "gathers of the candidates' rows through L1 (long_scoreboard) and issue; "
+                    "mma.sync tiles at a seventh of the tensor pipe",
+    "knn_join_tc": "latency and barriers: per-tile TMA gathers from L2 and the consumer "
                    "barriers; tensor pipe lightly used",
     "knn_merge": "latency: dependent pool loads and global atomics per node",
 }

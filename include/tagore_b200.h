@@ -27,7 +27,8 @@ enum {
 /* kNN join modes. CHOSEN: tensor-core screen + exact re-rank for rows up to
  * 1024 dims (one tile up to 128 dims, the tile accumulated over 64-dim blocks
  * from there; widths of 4 mod 8 on a zero-padded copy), the learned screen for
- * wider rows; PLAIN: every pair in exact FP32; LEARNED: the learned screen at
+ * wider rows, for rows below 16 dims and where the device has no room for the
+ * copy; PLAIN: every pair in exact FP32; LEARNED: the learned screen at
  * any width. */
 enum { TAGORE_KNN_CHOSEN = 0, TAGORE_KNN_PLAIN = 1, TAGORE_KNN_LEARNED = 2 };
 

@@ -455,7 +455,7 @@ __device__ void join_producer(TcSmem& s, const CUtensorMap& tmap, const float2* 
 // kept pairs exactly. Three blocks per SM (12 consumer warps) with one
 // 128-column accumulator each hide more latency than two blocks with two
 // accumulators each: 240 against 312 ms for ten joins at 1M x 128, K = 96, when that
-// was chosen; they take 105 ms now.
+// was chosen; they take 107 ms now.
 template <int D>
 __global__ void __launch_bounds__(kThreads, 3)
     k_join_tc(const __grid_constant__ CUtensorMap tmap, const float2* __restrict__ meta,

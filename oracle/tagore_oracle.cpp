@@ -217,7 +217,11 @@ uint32_t beam(const State& s, const uint32_t* G, const uint16_t* query, uint32_t
     rebuild_id2();
   }
   if (ring_count) *ring_count = curr;
-  return id[0];
+  // defined here: the beam's first node. With TOPM > K it has empty places, and they
+  // come first where every distance lies beyond kInfDis (the reference returns one)
+  for (uint32_t i = 0; i < topm; ++i)
+    if (id[i] != kInv) return id[i];
+  return start;
 }
 
 // Sort a candidate list by distance with the reference network and mark

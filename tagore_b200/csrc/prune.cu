@@ -397,7 +397,16 @@ __device__ uint32_t warp_beam(const uint32_t* __restrict__ G, const __half* __re
     to_explore = kInv;
   }
   if (ring_count) *ring_count = curr;
-  return bm.id[0];
+  if constexpr (kSolo) {
+    // The beam's first node. With TOPM > K the prefix has empty places, and they come
+    // first where every distance lies beyond their kInfDis.
+    for (uint32_t base = 0; base < topm; base += 32) {
+      const uint32_t j = base + lane;
+      const unsigned m = __ballot_sync(kFull, j < topm && bm.id[j] != kInv);
+      if (m) return bm.id[base + __ffs(m) - 1];
+    }
+  }
+  return start;
 }
 
 // Sort by distance with the reference network, then mark adjacent repeats

@@ -2,7 +2,8 @@
 
 The filter skips the node's own id only while it looks for the first kept
 candidate; behind a row equal to the node's it is a candidate like any other. So
-the kept sets of nodes with repeated vectors depend on where the id stands."""
+the kept sets of nodes with repeated vectors depend on where the id stands. Own ids in
+the rows, and distances around those of the empty places, take the same paths."""
 import numpy as np
 import pytest
 
@@ -59,6 +60,18 @@ def test_own_id_inside_the_row(capi, orc, dim, mode, metric, thre):
     half, ids, dis, center = graph(orc, gaussian(500, dim, 3), 32, 4)
     ids, dis = own_ids(ids, dis)
     run_pair(capi, orc, (half, ids, dis, center), 20, ("cfs", mode, metric), topm=40, thre=thre)
+
+
+@pytest.mark.parametrize("scale,topm", [(120.0, 30), (300.0, 24), (700.0, 16), (700.0, 30),
+                                        (3000.0, 64)])
+@pytest.mark.parametrize("mode,metric,thre", CFS)
+def test_distances_around_the_empty_places(capi, orc, mode, metric, thre, scale, topm):
+    # an unused place of the beam or of the list has the distance 1e7: these distances
+    # lie below it, around it and beyond it, those of the own ids too
+    half, ids, dis, center = graph(orc, gaussian(300, 64, 8, scale=scale), 24, 9)
+    ids, dis = own_ids(ids, dis)
+    ids[1::3, 0] = np.arange(len(ids))[1::3]
+    run_pair(capi, orc, (half, ids, dis, center), 20, ("cfs", mode, metric), topm=topm, thre=thre)
 
 
 @pytest.mark.parametrize("dim", [12, 128])

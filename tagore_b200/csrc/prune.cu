@@ -146,7 +146,9 @@ __device__ __forceinline__ float key_dis(uint64_t k) { return __uint_as_float((u
 
 // Merges the m entering entries, whose (distance, slot) keys sit in sm/sid
 // [0, m), into the sorted prefix [0, topm) by rank, through the staging
-// arrays. Returns false (nothing moved) when two merged positions 0..topm tie.
+// arrays. Returns false (nothing moved) when two merged positions 0..topm tie, or when
+// the prefix is out of order, as the network leaves it where distances are NaN: two
+// entries would take one place, and another keep whatever the staging held.
 template <bool kSolo, int E>
 __device__ __noinline__ bool beam_merge(Beam bm, uint32_t topm, uint32_t m, int lane) {
   uint64_t key[E];
@@ -163,8 +165,10 @@ __device__ __noinline__ bool beam_merge(Beam bm, uint32_t topm, uint32_t m, int 
   }
   __syncwarp();
   // merged rank: prefix i -> i + #(entering < A_i); entering q -> q + #(prefix <= B_q)
+  bool bad = false;
   for (uint32_t i = lane; i < topm; i += 32) {
     const float a = bm.dis[i];
+    bad |= i > 0 && !(bm.dis[i - 1] <= a);
     uint32_t lo = 0, hi = m;
     while (lo < hi) {
       const uint32_t mid = (lo + hi) >> 1;
@@ -199,9 +203,8 @@ __device__ __noinline__ bool beam_merge(Beam bm, uint32_t topm, uint32_t m, int 
     }
   }
   __syncwarp();
-  bool tie = false;
-  for (uint32_t p = lane + 1; p <= topm; p += 32) tie |= bm.sm[p] == bm.sm[p - 1];
-  if (__any_sync(kFull, tie)) return false;
+  for (uint32_t p = lane + 1; p <= topm; p += 32) bad |= bm.sm[p] == bm.sm[p - 1];
+  if (__any_sync(kFull, bad)) return false;
   for (uint32_t i = lane; i < topm; i += 32) {
     bm.dis[i] = bm.sm[i];
     bm.id[i] = bm.sid[i];

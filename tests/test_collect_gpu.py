@@ -36,3 +36,24 @@ def test_rows_out_of_order(capi, orc, mode, metric, thre):
 def test_widths_and_beams(capi, orc, dim, K, topm):
     run_pair(capi, orc, graph(orc, gaussian(400, dim, dim), K, 7), min(K, 40),
              ("cfs", "path", "dist"), topm=topm, thre=1.1)
+
+
+@pytest.mark.parametrize("K,topm", [(24, 16), (24, 40), (96, 64)])
+def test_nan_rows(capi, orc, K, topm):
+    # every ninth row is NaN: its distances stand anywhere in a beam that the network
+    # has sorted. Such a prune is a function of its input, of valid ids
+    x = gaussian(700, 32, 21)
+    x[::9, 5] = np.nan
+    ids, dis = orc.knn_input(gaussian(700, 32, 21), K, noise=0.3, seed=22)
+    dis = orc.dist_pairs(x, np.repeat(np.arange(700), K), ids.reshape(-1)).reshape(700, K)
+    center = gaussian(1, 32, 23)[0]
+    rows = []
+    for _ in range(2):
+        st = capi.State.from_host(ids, dis, x, center)
+        ep = capi.pruning_cfs(st, 20, "path", "dist", topm=topm, thre=1.1)
+        g = st.download(0).reshape(700, K)
+        st.free()
+        assert ep < 700 and (g[:, 0] < K).all()
+        assert all((r[1:1 + r[0]] < 700).all() for r in g)
+        rows.append(g)
+    assert np.array_equal(rows[0], rows[1])
